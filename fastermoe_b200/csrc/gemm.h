@@ -18,21 +18,23 @@ struct HostSegs {
 // Row range [lo, hi) of expert e, made safe for buffers of n_rows rows: the offsets come from
 // device memory that no host code has looked at, so a range is clamped to start no earlier than
 // the previous expert's end and to end no later than n_rows.  Valid offsets (non-decreasing,
-// last one <= n_rows) pass through unchanged.  Returns true when something had to be clamped.
-__device__ __forceinline__ bool safe_seg_range(const int64_t* __restrict__ off, const HostSegs& hs, int e, int64_t n_rows,
+// last one <= n_rows) pass through unchanged.  (Clamping range by range amounts to a running maximum, whose
+// loads do not wait for one another.)
+__device__ __forceinline__ void safe_seg_range(const int64_t* __restrict__ off, const HostSegs& hs, int e, int64_t n_rows,
                                                int64_t& lo, int64_t& hi) {
-    int64_t prev_hi = 0;
-    bool clamped = false;
-    for (int j = 0; j <= e; ++j) {
-        const int64_t raw_lo = hs.n ? (int64_t)hs.lo[j] : off[j], raw_hi = hs.n ? (int64_t)hs.hi[j] : off[j + 1];
-        lo = raw_lo < prev_hi ? prev_hi : raw_lo;
-        if (lo > n_rows) lo = n_rows;
-        hi = raw_hi < lo ? lo : raw_hi;
-        if (hi > n_rows) hi = n_rows;
-        clamped |= lo != raw_lo || hi != raw_hi;
-        prev_hi = hi;
+    int64_t before = 0, raw_lo, raw_hi;
+    if (hs.n) {
+        for (int j = 0; j < e; ++j) before = max(before, (int64_t)max(hs.lo[j], hs.hi[j]));
+        raw_lo = hs.lo[e];
+        raw_hi = hs.hi[e];
+    } else {
+#pragma unroll 8
+        for (int j = 0; j < e; ++j) before = max(before, off[j]);
+        raw_lo = off[e];
+        raw_hi = off[e + 1];
     }
-    return clamped;
+    lo = min(max(before, raw_lo), n_rows);
+    hi = min(max(lo, raw_hi), n_rows);
 }
 #endif
 

@@ -23,33 +23,6 @@ int check_common(int64_t n_rows, int64_t in_feat, int64_t out_feat, int n_expert
     return 0;
 }
 
-// out[e, c] = sum of grad_x[r, c] over the rows of expert e (plain kernel for the FFMA path).
-template <typename T>
-__global__ void colsum_rows_kernel(const T* __restrict__ gx, const int64_t* __restrict__ seg, const HostSegs hs,
-                                   T* __restrict__ out, int64_t n_rows, int64_t n_cols) {
-    const int e = blockIdx.y;
-    const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= n_cols) return;
-    int64_t lo, hi;
-    safe_seg_range(seg, hs, e, n_rows, lo, hi);
-    float s = 0.f;
-    for (int64_t r = lo; r < hi; ++r) s += to_float<T>(gx[r * n_cols + c]);
-    out[(int64_t)e * n_cols + c] = from_float<T>(s);
-}
-
-int colsum_rows(const LinearBwdArgs& a, cudaStream_t st) {
-    static const HostSegs none = {};
-    const HostSegs& hs = a.host_segs ? *a.host_segs : none;
-    dim3 grid((unsigned)ceil_div(a.in_feat, 128), (unsigned)a.n_expert);
-    switch (a.dtype) {
-        case FMOE_F32: colsum_rows_kernel<float><<<grid, 128, 0, st>>>((const float*)a.grad_x, a.seg_offsets, hs, (float*)a.grad_x_colsum, a.n_rows, a.in_feat); break;
-        case FMOE_F16: colsum_rows_kernel<__half><<<grid, 128, 0, st>>>((const __half*)a.grad_x, a.seg_offsets, hs, (__half*)a.grad_x_colsum, a.n_rows, a.in_feat); break;
-        default: colsum_rows_kernel<__nv_bfloat16><<<grid, 128, 0, st>>>((const __nv_bfloat16*)a.grad_x, a.seg_offsets, hs, (__nv_bfloat16*)a.grad_x_colsum, a.n_rows, a.in_feat); break;
-    }
-    FMOE_CHECK_LAUNCH();
-    return 0;
-}
-
 }  // namespace
 
 namespace fmoe {
@@ -61,9 +34,7 @@ int dispatch_linear_forward(const LinearArgs& a, cudaStream_t st) {
 int dispatch_linear_backward(const LinearBwdArgs& a, cudaStream_t st) {
     if (a.grad_x_colsum) FMOE_REQUIRE(a.grad_x, "linear_backward: column sums of grad_x requested without grad_x");
     if (!force_simt() && tc_backward_supported(a) && a.n_rows > 0) return tc_linear_backward(a, st);
-    if (int rc = simt_linear_backward(a, st)) return rc;
-    if (a.grad_x_colsum) return colsum_rows(a, st);   // the tensor-core kernel produces them itself
-    return 0;
+    return simt_linear_backward(a, st);
 }
 }  // namespace fmoe
 

@@ -77,6 +77,36 @@ def test_linear_forward_backward(fc, dtype, counts, fin, fout, bias):
     assert torch.equal(y, y2)
 
 
+@pytest.mark.parametrize("counts,fin,fout", [
+    ([127, 0, 129, 1], 36, 132),            # remainders of the 64-row and 128-column tiles, vectors of four
+    ([65, 63], 15, 131),                    # widths that are not multiples of four
+    ([3000, 0, 1, 2112], 132, 900),         # enough tiles for the 128-row form, ragged segments and columns
+    ([2600, 2601], 129, 1023),              # ... element by element
+])
+@pytest.mark.parametrize("offset", [0, 1])
+def test_fp32_products_at_tile_edges(fc, counts, fin, fout, offset):
+    """fp32 products against fp64.  ``offset``: operands one element past a 16-byte boundary.  Bound: a sum of k
+    products accumulated in fp32 is within k * 2^-24 * sum|a b| of the exact one (observed far below)."""
+    torch.manual_seed(fin + fout)
+    E, B = len(counts), sum(counts)
+
+    def mk(*shape):
+        flat = torch.randn(int(np.prod(shape)) + offset, device="cuda")
+        return flat[offset:].view(*shape)
+    x, w, b, gy = mk(B, fin), mk(E, fout, fin), mk(E, fout), mk(B, fout)
+    cnt = torch.tensor(counts, dtype=torch.int64)
+    y = fc.linear_forward(x, cnt, w, b)
+    gx, gw, gb = fc.linear_backward(gy, x, cnt, w, b)
+    p = 0
+    for e, c in enumerate(counts):
+        xe, we, ge = x[p:p + c].double(), w[e].double(), gy[p:p + c].double()
+        for got, want, mag, k in ((y[p:p + c], xe @ we.t() + b[e].double(), xe.abs() @ we.abs().t() + b[e].abs(), fin + 1),
+                                  (gx[p:p + c], ge @ we, ge.abs() @ we.abs(), fout),
+                                  (gw[e], ge.t() @ xe, ge.abs().t() @ xe.abs(), c), (gb[e], ge.sum(0), ge.abs().sum(0), c)):
+            assert ((got.double() - want).abs() <= max(k, 1) * 2.0 ** -24 * mag.double()).all()
+        p += c
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("act", ["relu", "gelu"])
 def test_fused_mlp_matches_autograd(fc, dtype, act):
