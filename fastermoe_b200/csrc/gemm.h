@@ -150,6 +150,12 @@ struct LinearBwdArgs {
 int simt_linear_forward(const LinearArgs& a, cudaStream_t st);
 int simt_linear_backward(const LinearBwdArgs& a, cudaStream_t st);
 
+// Widths on the 64-element grid of the token-major kernels.  Products that take part in an exchange (rows arriving,
+// or leaving as they are produced) need them: the form for other widths knows no peers.
+inline bool tc_grid_widths(int64_t in_feat, int64_t out_feat) {
+    return in_feat % 64 == 0 && out_feat % 64 == 0 && in_feat >= 256 && out_feat >= 256;
+}
+
 // Current FMOE_GEMM_* form (see fmoe_gemm_set_form).
 int gemm_form();
 

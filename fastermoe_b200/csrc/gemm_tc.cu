@@ -20,6 +20,9 @@
 // reads of DGRAD/WGRAD) are fetched as 64x64 boxes laid 8 KB apart, which is the
 // canonical MN-major layout of the UMMA shared-memory descriptor.
 //
+// Feature sizes off the 64-element grid (multiples of 8, at least 32) take a token-minor form of FWD and DGRAD, in
+// which the roles of the operands are exchanged (see Form); WGRAD takes them as it is.
+//
 // The work list is derived on the device from the expert segment offsets, so
 // the host never reads the counts.  Every mbarrier wait is bounded: on expiry
 // the kernel raises a status word, drains and exits (see fmoe_device_status).
@@ -38,7 +41,7 @@ constexpr int BM = 128, BN = 256, BK = 64;
 constexpr int A_BYTES = BM * BK * 2;    // 16 KB: the CTA's 128 rows of A
 constexpr int SUB_BYTES = 64 * BK * 2;  // one 64x64 box: 8 KB
 constexpr int RING_BYTES = 192 * 1024;  // operand ring of one CTA
-constexpr int MAX_STAGES = 6;
+constexpr int MAX_STAGES = 8;
 
 // One CTA per tile (128 x 256), or a pair of CTAs per tile (256 x 256, cta_group::2):
 // in a pair each CTA holds its own 128 rows of A and 128 of the 256 B columns, so
@@ -81,6 +84,7 @@ struct Params {
     int act;
     int accumulate;  // WGRAD only
     int is_bf16;
+    int tile_n, stages;   // token-minor form: tokens per tile, stages of the operand ring
     float* colsum;  // DGRAD: fp32 partial column sums of the output, one row per 32-row block, or null
     int tma_store;  // outputs have tensor maps: full 32-row blocks leave through TMA stores
     int* status;  // device status word
@@ -112,7 +116,7 @@ __device__ int g_status = 0;
 
 // Tensor maps of the outputs (box: 32 rows x 32 columns, 64-byte swizzle = the layout of the
 // epilogue's staging buffers): `out`, and the forward's second output (saved derivative).
-struct OutMaps { CUtensorMap out, out2; };
+struct OutMaps { CUtensorMap out, out2, b_full; };   // b_full: token-minor form, boxes of 128 tokens
 
 // ---- PTX wrappers ------------------------------------------------------------
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -247,6 +251,18 @@ __device__ __forceinline__ void tma_load_2d_pair(const CUtensorMap* map, uint32_
         ::"r"(smem_u32(dst)), "l"(map), "r"(bar_cluster), "r"(x), "r"(y)
         : "memory");
 }
+__device__ __forceinline__ void tma_load_3d(const CUtensorMap* map, unsigned long long* bar, void* dst, int x, int y, int z) {
+    asm volatile(
+        "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
+        ::"r"(smem_u32(dst)), "l"(map), "r"(smem_u32(bar)), "r"(x), "r"(y), "r"(z)
+        : "memory");
+}
+__device__ __forceinline__ void tma_load_3d_pair(const CUtensorMap* map, uint32_t bar_cluster, void* dst, int x, int y, int z) {
+    asm volatile(
+        "cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
+        ::"r"(smem_u32(dst)), "l"(map), "r"(bar_cluster), "r"(x), "r"(y), "r"(z)
+        : "memory");
+}
 // Bulk store of one staging buffer (smem, written by this warp) to the tile of `map` at (x, y).
 __device__ __forceinline__ void tma_store_2d(const CUtensorMap* map, const void* src, int x, int y) {
     asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%2, %3}], [%1];"
@@ -300,9 +316,9 @@ __device__ __forceinline__ uint64_t make_desc(uint32_t saddr, uint32_t lbo_bytes
 // Instruction descriptor, kind::f16: fp32 accumulate, A/B both bf16 or both fp16.
 //   [4,6) C format (1 = f32)  [7,10) A format  [10,13) B format (0 = f16, 1 = bf16)
 //   [15] A major (1 = MN)  [16] B major (1 = MN)  [17,23) N >> 3  [24,29) M >> 4
-__host__ __device__ constexpr uint32_t make_idesc(bool bf16, bool a_mn, bool b_mn, int m) {
+__host__ __device__ constexpr uint32_t make_idesc(bool bf16, bool a_mn, bool b_mn, int m, int n = BN) {
     return (1u << 4) | ((bf16 ? 1u : 0u) << 7) | ((bf16 ? 1u : 0u) << 10) | ((a_mn ? 1u : 0u) << 15) |
-           ((b_mn ? 1u : 0u) << 16) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(m >> 4) << 24);
+           ((b_mn ? 1u : 0u) << 16) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24);
 }
 
 // ---- packed fp32 arithmetic ----------------------------------------------------
@@ -422,21 +438,41 @@ __device__ __forceinline__ void stage_put(uint4* stage, int lane, const float* v
                        cvt_pack<BF16>(v[q * 8 + 4], v[q * 8 + 5]), cvt_pack<BF16>(v[q * 8 + 6], v[q * 8 + 7]));
     __syncwarp();
 }
-// staging -> global: rows [0, rows) of the block, CW columns starting at dst.
-__device__ __forceinline__ void stage_store(const uint4* stage, int lane, uint16_t* dst, size_t ld, int rows) {
+// staging -> global: rows [0, rows) and columns [0, cols) (a multiple of 8) of the block starting at dst.
+__device__ __forceinline__ void stage_store(const uint4* stage, int lane, uint16_t* dst, size_t ld, int rows, int cols) {
     constexpr int RPI = 32 / NCH;  // rows per instruction
     const int j = lane % NCH;
 #pragma unroll
     for (int it = 0; it < 32 / RPI; ++it) {
         const int row = it * RPI + lane / NCH;
-        if (row < rows) *reinterpret_cast<uint4*>(dst + (size_t)row * ld + j * 8) = stage[stage_slot(row, j)];
+        if (row < rows && j * 8 < cols) *reinterpret_cast<uint4*>(dst + (size_t)row * ld + j * 8) = stage[stage_slot(row, j)];
     }
     __syncwarp();
 }
-// CW values of this lane's own row (contiguous), or zeros when the row is absent.
-__device__ __forceinline__ void row_load(uint4* q, const uint16_t* src, bool valid) {
+// The first `cols` (a multiple of 8) of CW values of this lane's own row (contiguous), zeros elsewhere and when
+// the row is absent.
+__device__ __forceinline__ void row_load(uint4* q, const uint16_t* src, bool valid, int cols) {
 #pragma unroll
-    for (int i = 0; i < NCH; ++i) q[i] = valid ? __ldg(reinterpret_cast<const uint4*>(src) + i) : make_uint4(0, 0, 0, 0);
+    for (int i = 0; i < NCH; ++i) q[i] = valid && i * 8 < cols ? __ldg(reinterpret_cast<const uint4*>(src) + i) : make_uint4(0, 0, 0, 0);
+}
+
+// Token-minor accumulators: the lane holds one output column, v[j] belongs to row (token) j of the block.  The
+// 16-bit values go to the same staging layout, one column of 2-byte stores at a time (a warp's store fills 64
+// consecutive bytes of a row).
+template <bool BF16>
+__device__ __forceinline__ void stage_put_column(uint4* stage, int lane, const float* v) {
+    uint16_t* st = reinterpret_cast<uint16_t*>(stage);
+#pragma unroll
+    for (int j = 0; j < 32; j += 2) {
+        const uint32_t w = cvt_pack<BF16>(v[j], v[j + 1]);
+        st[stage_slot(j, lane >> 3) * 8 + (lane & 7)] = (uint16_t)(w & 0xffffu);
+        st[stage_slot(j + 1, lane >> 3) * 8 + (lane & 7)] = (uint16_t)(w >> 16);
+    }
+}
+// The lane's column of a staged block: value of row j.
+template <bool BF16>
+__device__ __forceinline__ float stage_get(const uint4* stage, int lane, int j) {
+    return cvt_in<BF16>(reinterpret_cast<const uint16_t*>(stage)[stage_slot(j, lane >> 3) * 8 + (lane & 7)]);
 }
 
 // ---- the spare warps' job when the product delivers its own input rows (GemmPushIn) ------------------
@@ -581,14 +617,21 @@ struct Tile {
 };
 
 // Tile of the CTA group; row0/rows span TILE_M rows (a CTA of a pair takes 128 of them).
-template <int MODE, int TILE_M>
+// Token-minor form: row0/rows are the tile's tokens (up to tile_n), col0 its first of TILE_M output columns.
+template <int MODE, int TILE_M, bool SWAP>
 __device__ __forceinline__ void locate(const Shared* sh, const Params& p, int tile, int& e_cursor, Tile& t) {
     while (tile >= sh->cum_tiles[e_cursor + 1]) ++e_cursor;
     const int local = tile - sh->cum_tiles[e_cursor];
-    const int nt = (p.n_out + BN - 1) / BN;
+    const int nt = SWAP ? (p.n_out + TILE_M - 1) / TILE_M : (p.n_out + BN - 1) / BN;
     t.e = e_cursor;
     const int lo = sh->seg_lo[e_cursor], hi = sh->seg_hi[e_cursor];
-    if (MODE == MODE_WGRAD) {
+    if (SWAP) {
+        t.row0 = lo + (local / nt) * p.tile_n;
+        t.rows = min(p.tile_n, hi - t.row0);
+        t.col0 = (local % nt) * TILE_M;
+        t.chunks = (p.n_contr + BK - 1) / BK;
+        t.m_lo = t.m_hi = 0;
+    } else if (MODE == MODE_WGRAD) {
         t.row0 = (local / nt) * TILE_M;
         t.rows = min(TILE_M, p.out_rows_per_expert - t.row0);
         t.col0 = (local % nt) * BN;
@@ -604,13 +647,18 @@ __device__ __forceinline__ void locate(const Shared* sh, const Params& p, int ti
     }
 }
 
-template <int MODE, bool BF16, bool CTA2>
+template <int MODE, bool BF16, bool CTA2, bool SWAP>
 __global__ void __launch_bounds__(THREADS, 1)
 grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                     const __grid_constant__ HostSegs hs, const __grid_constant__ OutMaps om,
                     const __grid_constant__ GemmRemoteOut ro, const __grid_constant__ GemmPushIn ps, const Params p) {
     using C = Cfg<CTA2>;
-    constexpr int STAGES = C::STAGES, STAGE_BYTES = C::STAGE_BYTES, TILE_M = C::TILE_M, B_COLS = C::B_COLS;
+    static_assert(!SWAP || MODE != MODE_WGRAD, "the weight gradient has no token-minor form");
+    constexpr int TILE_M = C::TILE_M, B_COLS = C::B_COLS;
+    const int STAGES = SWAP ? p.stages : C::STAGES;
+    const int STAGE_BYTES = SWAP ? A_BYTES + (CTA2 ? p.tile_n / 2 : p.tile_n) * BK * 2 : C::STAGE_BYTES;
+    // Token-minor form: tokens of a tile that are multiplied, a multiple of TOK_STEP (32 staged by each CTA).
+    constexpr int TOK_STEP = CTA2 ? 64 : 32;
     // Pairs: TMA completions of both CTAs go straight to the leader's barriers, so the MMA
     // issuer waits on one barrier and no warp of the second CTA sits in the critical path.
     // (The weight gradient's ragged contraction tail is then patched by the leader in both
@@ -652,7 +700,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
         // changed anything), so tile counts, scratch indices and stores stay in bounds.
         // One lane per expert and warp scans: all offsets are fetched at once (one thread walking them put about
         // 4 us in front of the first copy at 64 experts: six products of 16384 rows x 1024 x 512 took 216 us, 192 now).
-        const int nt = (p.n_out + BN - 1) / BN, last = (int)p.n_rows;
+        const int nt = SWAP ? (p.n_out + TILE_M - 1) / TILE_M : (p.n_out + BN - 1) / BN, last = (int)p.n_rows;
         constexpr int ROUNDS = MAX_EXPERTS_TC / 32;
         int64_t raw_lo[ROUNDS], raw_hi[ROUNDS];
 #pragma unroll
@@ -682,7 +730,8 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
             before = max(before, __shfl_sync(0xffffffffu, far, 31));
             const int lo = min(max(prev, c_lo), last), hi = max(lo, c_hi), rows = e < p.n_expert ? hi - lo : 0;
             clamped |= e < p.n_expert && (lo != raw_lo[i] || hi != raw_hi[i]);
-            const int mt = ((MODE == MODE_WGRAD ? p.out_rows_per_expert : rows) + TILE_M - 1) / TILE_M;
+            const int tile_rows = SWAP ? p.tile_n : TILE_M;
+            const int mt = ((MODE == MODE_WGRAD ? p.out_rows_per_expert : rows) + tile_rows - 1) / tile_rows;
             const int my_tiles = e < p.n_expert ? mt * nt : 0, my_blks = (rows + 31) >> 5;
             int t_incl = my_tiles, b_incl = my_blks;
 #pragma unroll
@@ -781,7 +830,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
             if (arriving) epoch = __ldcg(p.arr_seq) + 1;
             for (int tile = first_tile; tile < total_tiles && ok; tile += tile_step) {
                 Tile t;
-                locate<MODE, TILE_M>(sh, p, tile, e_cur, t);
+                locate<MODE, TILE_M, SWAP>(sh, p, tile, e_cur, t);
                 if (arriving && t.chunks > 0) {
                     const unsigned long long* my_flags = p.arr_flags + ((size_t)(epoch & 1) * 64 + lane) * 256;
                     // the flag of the expert that comes next was read while the previous tile was being loaded
@@ -808,6 +857,32 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                     if (!(ok = mbar_wait(&sh->empty[s], ph ^ 1, sh, p.status, 1))) break;
                     uint8_t* a_dst = tiles + s * STAGE_BYTES;
                     uint8_t* b_dst = a_dst + A_BYTES;
+                    if (SWAP) {
+                        // map_a: weights [expert][out][in] (three dimensions: rows and columns past an expert's
+                        // matrix read as zeros); map_b: tokens, boxes of 32 rows, only those that hold some.
+                        const int half = (t.rows + TOK_STEP - 1) / TOK_STEP * 32, boxes = half / 32, bytes = A_BYTES + boxes * 32 * BK * 2;
+                        const uint32_t bar = CTA2 ? map_to_cta(&sh->full[s], 0) : 0u;
+                        if (!CTA2) mbar_expect_tx(&sh->full[s], bytes);
+                        else if (cta == 0) mbar_expect_tx(&sh->full[s], 2 * bytes);
+                        const int col = t.col0 + my_row, tok = t.row0 + cta * half;
+                        if (MODE == MODE_FWD) {
+                            if (CTA2) tma_load_3d_pair(&map_a, bar, a_dst, ch * BK, col, t.e);
+                            else tma_load_3d(&map_a, &sh->full[s], a_dst, ch * BK, col, t.e);
+                        } else {
+#pragma unroll
+                            for (int j = 0; j < BM / 64; ++j) {
+                                if (CTA2) tma_load_3d_pair(&map_a, bar, a_dst + j * SUB_BYTES, col + j * 64, ch * BK, t.e);
+                                else tma_load_3d(&map_a, &sh->full[s], a_dst + j * SUB_BYTES, col + j * 64, ch * BK, t.e);
+                            }
+                        }
+                        if (CTA2 && half == 128) tma_load_2d_pair(&om.b_full, bar, b_dst, ch * BK, tok);
+                        else for (int b = 0; b < boxes; ++b) {
+                            if (CTA2) tma_load_2d_pair(&map_b, bar, b_dst + b * (32 * BK * 2), ch * BK, tok + b * 32);
+                            else tma_load_2d(&map_b, &sh->full[s], b_dst + b * (32 * BK * 2), ch * BK, tok + b * 32);
+                        }
+                        if (++s == STAGES) { s = 0; ph ^= 1; }
+                        continue;
+                    }
                     if (DIRECT) {
                         // Both CTAs' bytes are counted on the leader's barrier, which the MMA
                         // issuer waits on: no relay through the other CTA's warps.
@@ -860,8 +935,8 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
         }
     } else if (warp == 1) {
         // ---- MMA issuer -------------------------------------------------------
-        constexpr bool A_MN = MODE == MODE_WGRAD, B_MN = MODE != MODE_FWD;
-        constexpr uint32_t idesc = make_idesc(BF16, A_MN, B_MN, TILE_M);
+        constexpr bool A_MN = SWAP ? MODE == MODE_DGRAD : MODE == MODE_WGRAD, B_MN = !SWAP && MODE != MODE_FWD;
+        uint32_t idesc = make_idesc(BF16, A_MN, B_MN, TILE_M);
         // K-major: 8-row groups 1024 B apart, K advance 32 B per UMMA_K=16.
         // MN-major: 64-element column blocks 8 KB apart (leading), 8-row K groups 1024 B apart (stride),
         //           K advance 16 rows x 128 B = 2048 B.
@@ -873,7 +948,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
         const bool leader = cta == 0;
         for (int tile = first_tile; tile < total_tiles && ok; tile += tile_step) {
             Tile t;
-            locate<MODE, TILE_M>(sh, p, tile, e_cur, t);
+            locate<MODE, TILE_M, SWAP>(sh, p, tile, e_cur, t);
             if (t.chunks == 0) continue;
             if (DIRECT && !leader) continue;
             if (leader) {
@@ -881,12 +956,14 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                 tc_fence_after();
             }
             const uint32_t tmem_c = tmem_base + acc * BN;
+            if (SWAP) idesc = make_idesc(BF16, A_MN, B_MN, TILE_M, (t.rows + TOK_STEP - 1) / TOK_STEP * TOK_STEP);
             for (int ch = 0; ch < t.chunks; ++ch) {
                 if (!(ok = mbar_wait(&sh->full[s], ph, sh, p.status, 3))) break;
                 tc_fence_after();
                 uint8_t* a_src = tiles + s * STAGE_BYTES;
                 uint8_t* b_src = a_src + A_BYTES;
                 int k_steps = BK / 16;  // UMMA_K = 16 rows of the chunk per instruction
+                if (SWAP) k_steps = min(k_steps, (p.n_contr - ch * BK + 15) >> 4);   // (past the end both operands are zero)
                 if (MODE == MODE_WGRAD) {
                     // Rows of the chunk past the end of the expert's segment belong to the next
                     // expert (or are uninitialised).  K steps that lie entirely past the end are
@@ -946,7 +1023,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
         const int quarter = warp & 3;    // TMEM lanes [32*quarter, +32) are readable by this warp
         const int cgrp = (warp - FIRST_EPI_WARP) >> 2;  // which COLS_PER_WARP of the tile's 256 columns
         const int r = quarter * 32 + lane;
-        uint4* stage = reinterpret_cast<uint4*>(tiles + STAGES * STAGE_BYTES) + (warp - FIRST_EPI_WARP) * (STAGING_BYTES / 16);
+        uint4* stage = reinterpret_cast<uint4*>(tiles + RING_BYTES) + (warp - FIRST_EPI_WARP) * (STAGING_BYTES / 16);
         int e_cur = 0, acc = 0;
         uint32_t acc_ph = 0;
         bool ok = true;
@@ -954,7 +1031,121 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                                              CTA2 ? map_to_cta(&sh->tmem_empty[1], 0) : 0u};
         for (int tile = first_tile; tile < total_tiles && ok; tile += tile_step) {
             Tile t;
-            locate<MODE, TILE_M>(sh, p, tile, e_cur, t);
+            locate<MODE, TILE_M, SWAP>(sh, p, tile, e_cur, t);
+            if (SWAP) {
+                // This warp: 32 output columns (one per lane) and COLS_PER_WARP of the tile's tokens.
+                const size_t ld = (size_t)p.n_out;
+                const int col_lo = t.col0 + cta * BM + quarter * 32, cols = min(32, p.n_out - col_lo);
+                const bool active = cols > 0 && cgrp * COLS_PER_WARP < t.rows;
+                float bias = 0.f;
+                if (MODE == MODE_FWD && p.bias && active && lane < cols)
+                    bias = cvt_in<BF16>(__ldg((const uint16_t*)p.bias + (size_t)t.e * ld + col_lo + lane));
+                // pre-activation factor of a block: 4 lanes per row, 8 rows per instruction
+                const uint16_t* aux_src = MODE == MODE_DGRAD ? (const uint16_t*)p.act_pre : nullptr;
+                uint4 aux[NCH];
+                auto aux_load = [&](int tok, int rows) {
+#pragma unroll
+                    for (int it = 0; it < NCH; ++it) {
+                        const int row = it * 8 + (lane >> 2);
+                        aux[it] = row < rows && (lane & 3) * 8 < cols
+                                      ? __ldg(reinterpret_cast<const uint4*>(aux_src + (size_t)(tok + row) * ld + col_lo + (lane & 3) * 8))
+                                      : make_uint4(0, 0, 0, 0);
+                    }
+                };
+                if (aux_src && active) aux_load(t.row0 + cgrp * COLS_PER_WARP, min(32, t.rows - cgrp * COLS_PER_WARP));
+                if (!(ok = mbar_wait(&sh->tmem_full[acc], acc_ph, sh, p.status, 4))) break;
+                tc_fence_after();
+                const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) + acc * BN + cgrp * COLS_PER_WARP;
+                for (int c = 0; active && c < COLS_PER_WARP / CW; ++c) {
+                    const int tok0 = cgrp * COLS_PER_WARP + c * CW, rows = min(32, t.rows - tok0);
+                    if (rows <= 0) break;
+                    const int row0 = t.row0 + tok0;
+                    const bool bulk = p.tma_store && rows == 32;
+                    uint16_t* out_blk = (uint16_t*)p.out + (size_t)row0 * ld + col_lo;
+                    float v[CW];
+                    tc_ld32(taddr + c * CW, reinterpret_cast<uint32_t*>(v));
+                    if (c > 0 && aux_src) aux_load(row0, rows);
+                    tc_wait_ld();
+                    if (lane == 0) tma_store_wait_read();   // an earlier bulk store may still be reading the buffer
+                    __syncwarp();
+                    if (MODE == MODE_FWD) {
+                        const f32x2 b2 = pk1(bias);
+#pragma unroll
+                        for (int i = 0; i < CW / 2; ++i) unpk(add2(pk(v[2 * i], v[2 * i + 1]), b2), v[2 * i], v[2 * i + 1]);
+                        if (p.pre_out && p.act == FMOE_ACT_GELU) {
+                            float g[CW];
+#pragma unroll
+                            for (int i = 0; i < CW / 2; ++i) {
+                                f32x2 val, grad;
+                                gelu_pair<true>(pk(v[2 * i], v[2 * i + 1]), val, grad);
+                                unpk(val, v[2 * i], v[2 * i + 1]);
+                                unpk(grad, g[2 * i], g[2 * i + 1]);
+                            }
+                            stage_put_column<BF16>(stage, lane, g);
+                            __syncwarp();
+                            if (bulk) {
+                                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                                __syncwarp();
+                                if (lane == 0) {
+                                    tma_store_2d(&om.out2, stage, col_lo, row0);
+                                    tma_store_wait_read();      // the staging buffer is reused right away
+                                }
+                                __syncwarp();
+                            } else {
+                                stage_store(stage, lane, (uint16_t*)p.pre_out + (size_t)row0 * ld + col_lo, ld, rows, cols);
+                            }
+                        } else if (p.act == FMOE_ACT_GELU) {
+#pragma unroll
+                            for (int i = 0; i < CW / 2; ++i) {
+                                f32x2 val, grad;
+                                gelu_pair<false>(pk(v[2 * i], v[2 * i + 1]), val, grad);
+                                unpk(val, v[2 * i], v[2 * i + 1]);
+                            }
+                        } else if (p.act != FMOE_ACT_NONE) {
+#pragma unroll
+                            for (int i = 0; i < CW; ++i) v[i] = act_fast(v[i], p.act);
+                        }
+                    } else if (aux_src) {
+#pragma unroll
+                        for (int it = 0; it < NCH; ++it) stage[stage_slot(it * 8 + (lane >> 2), lane & 3)] = aux[it];
+                        __syncwarp();
+                        if (p.act == FMOE_ACT_GELU) {
+#pragma unroll
+                            for (int j = 0; j < CW; ++j) v[j] *= stage_get<BF16>(stage, lane, j);
+                        } else {
+#pragma unroll
+                            for (int j = 0; j < CW; ++j) v[j] *= saved_act_grad(stage_get<BF16>(stage, lane, j), p.act);
+                        }
+                        __syncwarp();
+                    }
+                    stage_put_column<BF16>(stage, lane, v);
+                    if (MODE == MODE_DGRAD && p.colsum) {
+                        // column sum of the (rounded) block: this lane's own column, read back from the staging buffer
+                        float sum = 0.f;
+#pragma unroll
+                        for (int j = 0; j < CW; ++j)
+                            if (j < rows) sum += stage_get<BF16>(stage, lane, j);
+                        const int blk = sh->blk_base[t.e] + ((row0 - sh->seg_lo[t.e]) >> 5);
+                        if (lane < cols) p.colsum[(size_t)blk * ld + col_lo + lane] = sum;
+                    }
+                    __syncwarp();
+                    if (bulk) {
+                        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                        __syncwarp();
+                        if (lane == 0) tma_store_2d(&om.out, stage, col_lo, row0);
+                    } else {
+                        stage_store(stage, lane, out_blk, ld, rows, cols);
+                    }
+                }
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) {
+                    if (CTA2) mbar_arrive_remote(tmem_empty_addr[acc]);
+                    else mbar_arrive(&sh->tmem_empty[acc]);
+                }
+                if (++acc == 2) { acc = 0; acc_ph ^= 1; }
+                continue;
+            }
             // this CTA's 128 rows of the tile
             t.row0 += cta * BM;
             t.rows = min(BM, t.rows - cta * BM);
@@ -1003,7 +1194,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
             if (MODE == MODE_DGRAD && p.act_pre) { aux_src = (const uint16_t*)p.act_pre + (row_off + r) * ld + col_lo; aux_row = row_ok; }
             if (MODE == MODE_WGRAD && p.accumulate) { aux_src = (const uint16_t*)p.out + (row_off + r) * ld + col_lo; aux_row = row_ok; }
             uint4 aux[NCH];
-            if (aux_src && active) row_load(aux, aux_src, aux_row);
+            if (aux_src && active) row_load(aux, aux_src, aux_row, p.n_out - col_lo);
             if (!(ok = mbar_wait(&sh->tmem_full[acc], acc_ph, sh, p.status, 4))) break;
             tc_fence_after();
             const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) + acc * BN + cgrp * COLS_PER_WARP;
@@ -1013,7 +1204,8 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                     uint32_t raw[CW];
                     tc_ld32(taddr + c * CW, raw);
                     if (CW == 64) tc_ld32(taddr + c * CW + 32, raw + 32);
-                    if (c > 0 && aux_src) row_load(aux, aux_src + c * CW, aux_row);
+                    const int cols = p.n_out - (col_lo + c * CW);   // (may exceed CW)
+                    if (c > 0 && aux_src) row_load(aux, aux_src + c * CW, aux_row, cols);
                     tc_wait_ld();
                     float* v = reinterpret_cast<float*>(raw);
                     const uint4* aq = aux;
@@ -1059,7 +1251,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                                 }
                                 __syncwarp();
                             } else {
-                                stage_store(stage, lane, (uint16_t*)p.pre_out + (row_off + quarter * 32) * ld + col_lo + c * CW, ld, rows_here);
+                                stage_store(stage, lane, (uint16_t*)p.pre_out + (row_off + quarter * 32) * ld + col_lo + c * CW, ld, rows_here, cols);
                             }
                         } else if (p.act == FMOE_ACT_GELU) {
 #pragma unroll
@@ -1149,7 +1341,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                             __syncwarp();
                             if (lane == 0) tma_store_2d(&om.out, stage, col_lo + c * CW, (int)row_off + quarter * 32);
                         } else {
-                            stage_store(stage, lane, out_blk + c * CW, ld, rows_here);
+                            stage_store(stage, lane, out_blk + c * CW, ld, rows_here, cols);
                         }
                     }
                 }
@@ -1244,6 +1436,25 @@ int make_map(CUtensorMap* map, const void* base, int64_t rows, int64_t cols, int
     return 0;
 }
 
+// The experts' weights [n_expert, rows, cols], box [box_rows, 64 cols] of one expert: what lies past an expert's
+// rows or columns reads as zeros (a 2-D map would run on into the next expert).
+int make_weight_map(CUtensorMap* map, const void* base, int n_expert, int64_t rows, int64_t cols, int box_rows, bool bf16) {
+    EncodeFn enc = get_encode();
+    if (!enc) return fail(FMOE_ERR_CUDA, "cuTensorMapEncodeTiled is not available from the driver");
+    cuuint64_t dims[3] = {(cuuint64_t)cols, (cuuint64_t)rows, (cuuint64_t)n_expert};
+    cuuint64_t strides[2] = {(cuuint64_t)cols * 2, (cuuint64_t)(rows * cols) * 2};
+    cuuint32_t box[3] = {(cuuint32_t)BK, (cuuint32_t)box_rows, 1};
+    cuuint32_t estr[3] = {1, 1, 1};
+    CUresult r = enc(map, bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3,
+                     const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                     CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                     CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS)
+        return fail(FMOE_ERR_CUDA, "cuTensorMapEncodeTiled failed (%d) for [%d, %lld, %lld] weights", (int)r, n_expert,
+                    (long long)rows, (long long)cols);
+    return 0;
+}
+
 // Output tensor [rows, cols] of 16-bit elements, box 32 x 32, 64-byte swizzle.
 int make_out_map(CUtensorMap* map, const void* base, int64_t rows, int64_t cols, bool bf16) {
     EncodeFn enc = get_encode();
@@ -1309,6 +1520,20 @@ bool use_pairs(int mode, int64_t n_rows, int n_expert, int64_t n_out) {
     return n_rows >= (int64_t)512 * n_expert && pair_tiles >= 2 * (sm_count() / 2);
 }
 
+// Form of a forward or input-gradient product.  Token-major: tokens are the 128 (pairs: 256) rows of the tile,
+// 256 output columns.  Token-minor: 128 (pairs: 256) output columns are the tile's rows and up to tile_n tokens its
+// columns, in steps of 32 (pairs: 64).  Its three-dimensional weight map ends at each expert's rows, which lets widths
+// off the 64-element grid run on the tensor cores at all; on the grid it is the slower one (16384 rows of 32 skewed
+// experts, 2048 x 8192: 536 us token-major, 613 token-minor; 184 rows of 13: 75 and 83), so widths alone decide.
+// Off the grid, 3998 rows of six experts, 200 x 712: six products took 460 us on the FFMA pipe, 76 here.
+// tile_n: 64 tokens leave eight stages for streaming weights when experts have few rows; above 32 rows on average
+// pairs with 256 tokens, which pull fewer operand bytes per flop.
+struct Form { bool swap, pair; int tile_n; };
+Form pick_form(int mode, int64_t n_rows, int n_expert, int64_t n_out, int64_t n_contr) {
+    if (tc_grid_widths(n_contr, n_out)) return Form{false, use_pairs(mode, n_rows, n_expert, n_out), 0};
+    const bool pair = n_rows > (int64_t)32 * n_expert;
+    return Form{true, pair, pair ? 256 : 64};
+}
 // CTAs the persistent GEMM grids may use: all SMs, or fewer (FMOE_B200_GEMM_SMS=n, or
 // fmoe_gemm_set_sm_limit) to leave SMs to kernels that run beside them on other streams.
 int cta_cap() {
@@ -1323,13 +1548,18 @@ int cta_cap() {
     return std::max(cap, 2);
 }
 
+int ring_stages(const Form& f) { return std::min<int>(MAX_STAGES, RING_BYTES / (A_BYTES + (f.pair ? f.tile_n / 2 : f.tile_n) * BK * 2)); }
+int64_t swap_tiles(const Form& f, int64_t n_rows, int n_expert, int64_t n_out) {
+    return (ceil_div(n_rows, f.tile_n) + n_expert) * ceil_div(n_out, f.pair ? 256 : BM);
+}
+
 const GemmRemoteOut kNoRemote = {};
 const GemmPushIn kNoPush = {};
 
-template <int MODE, bool CTA2>
+template <int MODE, bool CTA2, bool SWAP = false>
 int launch(const CUtensorMap& ma, const CUtensorMap& mb, const HostSegs* hsp, const Params& p_in, int64_t max_tiles,
            int64_t out_rows, cudaStream_t st, int reserve_sms = 0, const GemmRemoteOut* rop = nullptr,
-           const GemmPushIn* psp = nullptr) {
+           const GemmPushIn* psp = nullptr, const CUtensorMap* b_full = nullptr) {
     const GemmRemoteOut& ro = rop ? *rop : kNoRemote;
     const GemmPushIn& ps = psp ? *psp : kNoPush;
     reserve_sms = (reserve_sms + 1) / 2 * 2;      // the kernel beside this one occupies whole SM pairs
@@ -1338,6 +1568,7 @@ int launch(const CUtensorMap& ma, const CUtensorMap& mb, const HostSegs* hsp, co
     static_assert(CW == 32, "the output tensor maps assume 32-column staging buffers");
     OutMaps om;
     memset(&om, 0, sizeof(om));
+    if (b_full) om.b_full = *b_full;
     p.tma_store = 0;
     if (out_rows > 0 && p.out && ro.enabled != 1) {
         if (int rc = make_out_map(&om.out, p.out, out_rows, p.n_out, p.is_bf16 != 0)) return rc;
@@ -1346,7 +1577,7 @@ int launch(const CUtensorMap& ma, const CUtensorMap& mb, const HostSegs* hsp, co
         }
         p.tma_store = 1;
     }
-    auto kern = p.is_bf16 ? grouped_gemm_kernel<MODE, true, CTA2> : grouped_gemm_kernel<MODE, false, CTA2>;
+    auto kern = p.is_bf16 ? grouped_gemm_kernel<MODE, true, CTA2, SWAP> : grouped_gemm_kernel<MODE, false, CTA2, SWAP>;
     FMOE_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_BYTES));
     cudaLaunchConfig_t cfg = {};
     cfg.blockDim = dim3(THREADS);
@@ -1385,8 +1616,8 @@ int launch(const CUtensorMap& ma, const CUtensorMap& mb, const HostSegs* hsp, co
 bool aligned16(const void* p) { return ((uintptr_t)p & 15) == 0; }
 
 bool shape_ok(int64_t n_rows, int64_t in_feat, int64_t out_feat, int n_expert, int dtype) {
-    return (dtype == FMOE_BF16 || dtype == FMOE_F16) && n_expert <= MAX_EXPERTS_TC && in_feat % 64 == 0 &&
-           out_feat % 64 == 0 && in_feat >= 256 && out_feat >= 256 && n_rows > 0 && n_rows < ((int64_t)1 << 31) &&
+    return (dtype == FMOE_BF16 || dtype == FMOE_F16) && n_expert <= MAX_EXPERTS_TC && in_feat % 8 == 0 &&
+           out_feat % 8 == 0 && in_feat >= 32 && out_feat >= 32 && n_rows > 0 && n_rows < ((int64_t)1 << 31) &&
            (int64_t)n_expert * out_feat < ((int64_t)1 << 31);
 }
 
@@ -1543,15 +1774,28 @@ size_t tc_backward_scratch_bytes(int64_t n_rows, int64_t in_feat, int64_t, int n
 int tc_linear_forward(const LinearArgs& a, cudaStream_t st) {
     const bool bf16 = a.dtype == FMOE_BF16;
     CUtensorMap ma, mb;
-    if (int rc = make_map(&ma, a.x, a.n_rows, a.in_feat, BM, bf16)) return rc;
-    // Pairs of CTAs (256-row tiles) once there is enough work for them; each CTA of a
-    // pair stages 128 of the tile's 256 weight rows.
-    const bool pair = use_pairs(MODE_FWD, a.n_rows, a.n_expert, a.out_feat);
-    if (int rc = make_map(&mb, a.weight, (int64_t)a.n_expert * a.out_feat, a.in_feat, pair ? 128 : BN, bf16)) return rc;
+    const Form form = pick_form(MODE_FWD, a.n_rows, a.n_expert, a.out_feat, a.in_feat);
+    // Pairs of CTAs once there is enough work for them; each CTA of a pair stages half of the tile's columns.
+    const bool pair = form.pair;
+    if (form.swap) {
+        if (int rc = make_weight_map(&ma, a.weight, a.n_expert, a.out_feat, a.in_feat, BM, bf16)) return rc;
+        if (int rc = make_map(&mb, a.x, a.n_rows, a.in_feat, 32, bf16)) return rc;
+    } else {
+        if (int rc = make_map(&ma, a.x, a.n_rows, a.in_feat, BM, bf16)) return rc;
+        if (int rc = make_map(&mb, a.weight, (int64_t)a.n_expert * a.out_feat, a.in_feat, pair ? 128 : BN, bf16)) return rc;
+    }
     Params p{};
     p.seg = a.seg_offsets; p.n_expert = a.n_expert; p.n_out = (int)a.out_feat; p.n_contr = (int)a.in_feat;
     p.w_rows = (int)a.out_feat; p.out = a.y; p.pre_out = a.pre_act; p.bias = a.bias; p.act = a.activation;
     p.is_bf16 = bf16; p.status = status_ptr(); p.n_rows = a.n_rows;
+    if (form.swap) {
+        p.tile_n = form.tile_n; p.stages = ring_stages(form);
+        const int64_t tiles = swap_tiles(form, a.n_rows, a.n_expert, a.out_feat);
+        CUtensorMap mf;
+        if (int rc = make_map(&mf, a.x, a.n_rows, a.in_feat, 128, bf16)) return rc;
+        return pair ? launch<MODE_FWD, true, true>(ma, mb, a.host_segs, p, tiles, a.n_rows, st, 0, nullptr, nullptr, &mf)
+                    : launch<MODE_FWD, false, true>(ma, mb, a.host_segs, p, tiles, a.n_rows, st);
+    }
     const int tile_m = pair ? 256 : BM;
     const int64_t max_tiles = (ceil_div(a.n_rows, tile_m) + a.n_expert) * ceil_div(a.out_feat, BN);
     int reserve = 0;
@@ -1621,8 +1865,14 @@ int tc_linear_backward(const LinearBwdArgs& a, cudaStream_t st) {
     }
     if (a.grad_x && a.n_rows > 0) {
         CUtensorMap ma, mb;
-        if (int rc = make_map(&ma, a.grad_y, a.n_rows, a.out_feat, BM, bf16)) return rc;
-        if (int rc = make_map(&mb, a.weight, (int64_t)a.n_expert * a.out_feat, a.in_feat, 64, bf16)) return rc;
+        const Form form = pick_form(MODE_DGRAD, a.n_rows, a.n_expert, a.in_feat, a.out_feat);
+        if (form.swap) {
+            if (int rc = make_weight_map(&ma, a.weight, a.n_expert, a.out_feat, a.in_feat, 64, bf16)) return rc;
+            if (int rc = make_map(&mb, a.grad_y, a.n_rows, a.out_feat, 32, bf16)) return rc;
+        } else {
+            if (int rc = make_map(&ma, a.grad_y, a.n_rows, a.out_feat, BM, bf16)) return rc;
+            if (int rc = make_map(&mb, a.weight, (int64_t)a.n_expert * a.out_feat, a.in_feat, 64, bf16)) return rc;
+        }
         Params p{};
         p.seg = a.seg_offsets; p.n_expert = a.n_expert; p.n_out = (int)a.in_feat; p.n_contr = (int)a.out_feat;
         p.w_rows = (int)a.out_feat; p.out = a.grad_x; p.act_pre = a.act_pre; p.act = a.activation;
@@ -1632,7 +1882,7 @@ int tc_linear_backward(const LinearBwdArgs& a, cudaStream_t st) {
                          "linear_backward: column sums of grad_x need the scratch buffer of fmoe_linear_scratch_bytes");
             p.colsum = (float*)a.scratch;
         }
-        const bool pair = use_pairs(MODE_DGRAD, a.n_rows, a.n_expert, a.in_feat);
+        const bool pair = form.pair;
         const int64_t max_tiles = (ceil_div(a.n_rows, pair ? 256 : BM) + a.n_expert) * ceil_div(a.in_feat, BN);
         int reserve = 0;
         if (arriving && !closed) {
@@ -1644,7 +1894,14 @@ int tc_linear_backward(const LinearBwdArgs& a, cudaStream_t st) {
             p.done = a.done->done; p.done_expected = a.done->expected; p.done_ready = a.done->ready;
             reserve = std::max(reserve, a.done->reserve_sms);
         }
-        if (int rc = pair ? launch<MODE_DGRAD, true>(ma, mb, a.host_segs, p, max_tiles, a.n_rows, st, reserve, a.remote, a.push)
+        if (form.swap) {
+            p.tile_n = form.tile_n; p.stages = ring_stages(form);
+            const int64_t tiles = swap_tiles(form, a.n_rows, a.n_expert, a.in_feat);
+            CUtensorMap mf;
+            if (int rc = make_map(&mf, a.grad_y, a.n_rows, a.out_feat, 128, bf16)) return rc;
+            if (int rc = pair ? launch<MODE_DGRAD, true, true>(ma, mb, a.host_segs, p, tiles, a.n_rows, st, 0, nullptr, nullptr, &mf)
+                              : launch<MODE_DGRAD, false, true>(ma, mb, a.host_segs, p, tiles, a.n_rows, st)) return rc;
+        } else if (int rc = pair ? launch<MODE_DGRAD, true>(ma, mb, a.host_segs, p, max_tiles, a.n_rows, st, reserve, a.remote, a.push)
                           : launch<MODE_DGRAD, false>(ma, mb, a.host_segs, p, max_tiles, a.n_rows, st, reserve, a.remote, a.push))
             return rc;
         if (!closed) {

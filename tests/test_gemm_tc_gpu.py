@@ -315,3 +315,82 @@ def test_input_gradient_column_sums(fc, dtype, form):
         else:
             torch.testing.assert_close(cs.float(), want, rtol=2e-2, atol=4 * 2.0 ** -9 * rms)
     assert device_status() == 0
+
+
+TOKEN_MINOR = [
+    # few tokens per expert (one CTA per tile): edges of the 32-token steps, experts without any
+    ([1, 31, 32, 33, 0, 63, 64, 65], 256, 384),
+    ([3, 0, 0, 1], 2048, 1024),
+    # pairs of CTAs: edges of the 64-token steps and of the 256-token tiles
+    ([255, 256, 257, 0, 1, 129], 512, 256),
+    ([700, 37], 256, 832),
+    # widths off the 64-element grid, the smallest ones, columns that end inside a 32-column block
+    ([100, 0, 29, 300], 200, 712),
+    ([5, 70], 32, 40),
+    ([33, 95, 64], 264, 72),
+    ([1300, 1, 1500], 136, 328),
+]
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("counts,fin,fout", TOKEN_MINOR)
+def test_token_minor_products(fc, dtype, counts, fin, fout):
+    """Forward (bias, GELU with its saved derivative), input gradient (with column sums) and weight gradient, against
+    fp32.  Rows past the segments hold NaNs and the expert after each used one holds infinities: neither may show."""
+    from fastermoe_b200 import _lib
+    torch.manual_seed(sum(counts) + fin + fout)
+    counts = [c for n in counts for c in (n, 0)]            # every other expert has no rows, and infinite weights
+    E, B, pad = len(counts), sum(counts), 3
+    x = torch.full((B + pad, fin), float("nan"), device="cuda", dtype=dtype)
+    gy = torch.full((B + pad, fout), float("nan"), device="cuda", dtype=dtype)
+    x[:B], gy[:B] = torch.randn(B, fin, device="cuda").to(dtype), torch.randn(B, fout, device="cuda").to(dtype)
+    w = ((torch.rand(E, fout, fin, device="cuda") * 2 - 1) / np.sqrt(fin)).to(dtype)
+    b = ((torch.rand(E, fout, device="cuda") * 2 - 1) / np.sqrt(fin)).to(dtype)
+    saved = torch.rand(B + pad, fin, device="cuda").to(dtype)
+    w[1::2] = float("inf")
+    off = torch.tensor(np.concatenate([[0], np.cumsum(counts)]), dtype=torch.int64, device="cuda")
+    y, pre = fc.linear_forward_act(x, off, w, b, _lib.ACT_GELU, want_pre=True)
+    plain, _ = fc.linear_forward_act(x, off, w, None, _lib.ACT_NONE)
+    gx, gw, gb, cs = fc.linear_backward_act(gy, x, off, w, saved, _lib.ACT_GELU, want_gx_colsum=True)
+    assert device_status() == 0
+    p = 0
+    for e, c in enumerate(counts):
+        xe, ge = x[p:p + c].float(), gy[p:p + c].float()
+        if c:
+            z = xe @ w[e].float().t()
+            close(plain[p:p + c], z)
+            zb = (z + b[e].float()).requires_grad_(True)
+            act = torch.nn.functional.gelu(zb)
+            close(y[p:p + c], act.detach())
+            close(pre[p:p + c], torch.autograd.grad(act.sum(), zb)[0])
+            close(gx[p:p + c], (ge @ w[e].float()) * saved[p:p + c].float())
+            # sums of the rounded rows
+            want = gx[p:p + c].float().sum(0)
+            torch.testing.assert_close(cs[e].float(), want, rtol=2e-2, atol=2.0 ** -8 * float(want.abs().max()))
+        close(gw[e], ge.t() @ xe)
+        close(gb[e], ge.sum(0))
+        p += c
+
+
+@pytest.mark.parametrize("act", ["relu", "none"])
+def test_token_minor_epilogues(fc, act):
+    """ReLU forward and backward and the plain products at a ragged size, against fp32."""
+    from fastermoe_b200 import _lib
+    torch.manual_seed(5)
+    counts, fin, fout = [40, 0, 97], 328, 200
+    code = {"relu": _lib.ACT_RELU, "none": _lib.ACT_NONE}[act]
+    E, B = len(counts), sum(counts)
+    x, gy = torch.randn(B, fin, device="cuda").bfloat16(), torch.randn(B, fout, device="cuda").bfloat16()
+    w = ((torch.rand(E, fout, fin, device="cuda") * 2 - 1) / np.sqrt(fin)).bfloat16()
+    b = torch.randn(E, fout, device="cuda").bfloat16()
+    saved = torch.randn(B, fin, device="cuda").relu().bfloat16()
+    off = torch.tensor(np.concatenate([[0], np.cumsum(counts)]), dtype=torch.int64, device="cuda")
+    y, _ = fc.linear_forward_act(x, off, w, b, code)
+    gx, _, _ = fc.linear_backward_act(gy, x, off, w, saved if act == "relu" else None, code)
+    p = 0
+    for e, c in enumerate(counts):
+        z = x[p:p + c].float() @ w[e].float().t() + b[e].float()
+        close(y[p:p + c], z.relu() if act == "relu" else z)
+        g = gy[p:p + c].float() @ w[e].float()
+        close(gx[p:p + c], g * (saved[p:p + c].float() > 0) if act == "relu" else g)
+        p += c
