@@ -41,6 +41,14 @@ class FusedGeometry(ctypes.Structure):
     _fields_ = [("n_steps", c_int32), ("gran", c_int32), ("global_rows", c_int64), ("shadow_rows", c_int64)]
 
 
+class MoeMlp(ctypes.Structure):
+    """Mirror of fmoe_moe_mlp_t."""
+    _fields_ = ([(n, c_void_p) for n in ("inp", "gate_idx", "score", "w1", "b1", "w2", "b2", "index", "rows", "out", "grad_out",
+                                         "grads", "grad_inp", "grad_score", "gw1", "gb1", "gw2", "gb2")] +
+                [(n, c_int64) for n in ("n_tokens", "d_model", "d_hidden")] +
+                [(n, c_int32) for n in ("top_k", "n_expert", "dtype", "activation", "keep", "reserved")])
+
+
 class MlpParams(ctypes.Structure):
     """Mirror of fmoe_mlp_params_t."""
     _fields_ = [(n, c_void_p) for n in ("w1", "w2", "b1", "b2", "gw1", "gw2", "gb1", "gb2")]
@@ -89,6 +97,9 @@ _SIGS = {
     "fmoe_linear_forward": (I32, [P, P, P, P, P, P, I64, I64, I64, I32, I32, I32, P]),
     "fmoe_linear_backward": (I32, [P, P, P, P, P, P, P, P, I64, I64, I64, I32, I32, I32, I32, P, P]),
     "fmoe_linear_backward_colsum": (I32, [P, P, P, P, P, P, P, P, P, I64, I64, I64, I32, I32, I32, I32, P, P]),
+    "fmoe_moe_mlp_bytes": (I32, [P, P, P, P]),
+    "fmoe_moe_mlp_forward": (I32, [P, P]),
+    "fmoe_moe_mlp_backward": (I32, [P, P]),
     "fmoe_comm_unique_id": (I32, [P]),
     "fmoe_comm_init": (I32, [P, I32, I32, I32, POINTER(c_void_p)]),
     "fmoe_comm_destroy": (I32, [P]),

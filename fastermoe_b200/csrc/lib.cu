@@ -42,6 +42,7 @@ extern "C" size_t fmoe_abi_sizeof(const char* struct_name) {
     if (!strcmp(struct_name, "fmoe_peer_seg_t")) return sizeof(fmoe_peer_seg_t);
     if (!strcmp(struct_name, "fmoe_arrival_t")) return sizeof(fmoe_arrival_t);
     if (!strcmp(struct_name, "fmoe_mlp_params_t")) return sizeof(fmoe_mlp_params_t);
+    if (!strcmp(struct_name, "fmoe_moe_mlp_t")) return sizeof(fmoe_moe_mlp_t);
     if (!strcmp(struct_name, "fmoe_fused_geometry_t")) return sizeof(fmoe_fused_geometry_t);
     return 0;
 }

@@ -16,7 +16,9 @@ reference's extension; they are the fused forms the layer in this package uses
 (bucketing in one call, permutation kernels, gate-score combine, activation
 fused into the expert GEMMs).
 """
+import contextlib
 import ctypes
+import functools
 import os
 import threading
 
@@ -56,6 +58,11 @@ class Profile:
 
 
 _profile = None
+
+
+def profiling():
+    """True while a Profile is installed: calls are then made operator by operator."""
+    return _profile is not None
 
 
 def set_profile(p):
@@ -103,7 +110,7 @@ def device_status(device=None):
     """The status word of ``device`` (0: no bounded wait expired, no offsets were clamped).
     Waits for the work queued on the device."""
     st = ctypes.c_int32(0)
-    with torch.cuda.device(device):
+    with _device_of(device):
         check(lib.fmoe_device_status(ctypes.byref(st)), "device_status")
     return st.value
 
@@ -113,7 +120,7 @@ def check_status(device=None):
     an expired bounded wait (results of that step are incomplete) or clamped segment offsets."""
     v = device_status(device)
     if v:
-        with torch.cuda.device(device):
+        with _device_of(device):
             lib.fmoe_device_status_clear()
         what = []
         if v & 15:
@@ -139,8 +146,19 @@ def _ptr(t):
     return ctypes.c_void_p(t.data_ptr()) if t is not None else None
 
 
-def _stream(device=None):
-    return ctypes.c_void_p(torch.cuda.current_stream(device).cuda_stream)
+_NO_SWITCH = contextlib.nullcontext()
+
+
+def _device_of(device):
+    """torch.cuda.device(device), without its cost when that device is current already."""
+    if isinstance(device, torch.device) and device.index is not None and device.index == torch.cuda.current_device():
+        return _NO_SWITCH
+    return torch.cuda.device(device)
+
+
+def _stream():
+    """The current device's current stream."""
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
 
 
 def _check_cuda(*tensors):
@@ -169,7 +187,7 @@ def expert_count(gate_idx, expert_count):
     """Adds the histogram of ``gate_idx`` (int64, -1 ignored) into ``expert_count`` (int32)."""
     _check_cuda(gate_idx, expert_count)
     assert gate_idx.dtype == torch.int64 and expert_count.dtype == torch.int32
-    with torch.cuda.device(gate_idx.device):
+    with _device_of(gate_idx.device):
         _run("expert_count", lib.fmoe_expert_count, _ptr(gate_idx), _ptr(expert_count), gate_idx.numel(),
                                     expert_count.numel(), _stream())
 
@@ -179,7 +197,7 @@ def assign_pos(cum_count, gate, pos):
     _check_cuda(cum_count, gate, pos)
     assert cum_count.dtype == torch.int32 and gate.dtype == torch.int64 and pos.dtype == torch.int64
     n, e = gate.numel(), cum_count.numel()
-    with torch.cuda.device(gate.device):
+    with _device_of(gate.device):
         scratch = _routing_scratch(n, e, gate.device)
         _run("assign_pos", lib.fmoe_assign_pos, _ptr(cum_count), _ptr(gate), _ptr(pos), n, e, _ptr(scratch),
                                   _stream())
@@ -195,7 +213,7 @@ def limit_by_capacity(expert_count, capacity, n_expert, n_worker):
     assert expert_count.dtype == torch.int64 and capacity.dtype == torch.int32
     assert expert_count.numel() == n_expert * n_worker and capacity.numel() == n_expert
     out = torch.empty_like(expert_count)
-    with torch.cuda.device(expert_count.device):
+    with _device_of(expert_count.device):
         _run("limit_by_capacity", lib.fmoe_limit_by_capacity, _ptr(expert_count), _ptr(capacity), _ptr(out), n_expert,
                                          n_worker, _stream())
     return out
@@ -208,7 +226,7 @@ def prune_gate_by_capacity(gate_idx, expert_count, n_expert, n_worker):
     assert expert_count.numel() == n_expert * n_worker
     out = torch.empty_like(gate_idx)
     n, e = gate_idx.numel(), expert_count.numel()
-    with torch.cuda.device(gate_idx.device):
+    with _device_of(gate_idx.device):
         scratch = _routing_scratch(n, e, gate_idx.device)
         _run("prune_gate_by_capacity", lib.fmoe_prune_gate_by_capacity, _ptr(gate_idx), _ptr(out), _ptr(expert_count), n, e,
                                               _ptr(scratch), _stream())
@@ -316,7 +334,7 @@ def ensure_nccl(group, t):
         if world > 1 and os.environ.get("FMOE_B200_PEER", "1") != "0":
             slot = int(os.environ.get("FMOE_B200_PEER_SLOT_MB", "256")) << 20
             pool = int(os.environ.get("FMOE_B200_PEER_POOL_MB", "2048")) << 20
-            with torch.cuda.device(dev):
+            with _device_of(dev):
                 _run("peer_enable", lib.fmoe_peer_enable, handle, slot, pool, _stream())
 
 
@@ -350,7 +368,7 @@ def expert_exchange(local_expert_count, n_expert, n_workers):
     aec = local_expert_count.new_empty((n_workers, n_workers, n_expert))
     agec = local_expert_count.new_empty((n_workers, n_workers, n_expert))
     gec = torch.empty_like(local_expert_count)
-    with torch.cuda.device(dev):
+    with _device_of(dev):
         _run("expert_exchange", lib.fmoe_expert_exchange, _comm(dev), _ptr(local_expert_count), _ptr(aec), _ptr(agec),
                                        _ptr(gec), n_expert, n_workers, _stream())
     return [aec, agec, gec]
@@ -387,7 +405,7 @@ def _global_move(fn, name, buf, local_expert_count, global_expert_count, stored_
     # (allocated on every rank, also one that receives nothing: all ranks must use the same form)
     staging = (buf.new_empty((max(int(expert_rows), 1), buf.shape[1]))
                if os.environ.get("FMOE_B200_EXCHANGE") != "split" else None)
-    with torch.cuda.device(buf.device):
+    with _device_of(buf.device):
         _run(name, fn, _comm(buf.device), _ptr(buf), _ptr(out), _ptr(lec), _ptr(gec), _ptr(st), buf.shape[0],
              batch_size, row_bytes, n_expert, n_workers, _ptr(staging), _stream())
     return out
@@ -491,7 +509,7 @@ def _peer_move(fn, name, buf, table, stored_models, batch_size, n_expert, n_work
     tab, st = _host_i64(table.reshape(-1)), _host_flags(stored_models)
     assert tab.numel() == n_workers * n_workers * n_expert
     out = _recv_empty(buf, batch_size)
-    with torch.cuda.device(buf.device):
+    with _device_of(buf.device):
         ok = _run(name, fn, _comm(buf.device), _ptr(buf), _ptr(out), _ptr(tab), _ptr(st), buf.shape[0], batch_size,
                   buf.shape[1] * buf.element_size(), n_expert, n_workers, _stream(), soft=True)
     return out if ok else None
@@ -557,7 +575,7 @@ def peer_plan_exchange(local_expert_count, stored_models, cap_rows, n_expert):
     assert local_expert_count.numel() == n_expert * world
     plan = _plan_buffer(n_expert, world, dev)
     st = stored_models.view(torch.uint8) if stored_models is not None and stored_models.dtype == torch.bool else stored_models
-    with torch.cuda.device(dev):
+    with _device_of(dev):
         ok = _run("peer_plan", lib.fmoe_peer_plan_exchange, _comm(dev), _ptr(local_expert_count), _ptr(st), int(cap_rows),
                   _ptr(plan), n_expert, _stream(), soft=True)
     return PeerPlan(plan, n_expert, world) if ok else None
@@ -570,7 +588,7 @@ def peer_plan_from_table(all_expert_count, stored_models, rank, n_expert, n_work
     assert all_expert_count.dtype == torch.int64 and all_expert_count.numel() == n_workers * n_workers * n_expert
     plan = _plan_buffer(n_expert, n_workers, dev)
     st = stored_models.view(torch.uint8) if stored_models is not None and stored_models.dtype == torch.bool else stored_models
-    with torch.cuda.device(dev):
+    with _device_of(dev):
         _run("peer_plan", lib.fmoe_peer_plan_from_table, _ptr(all_expert_count), _ptr(st), _ptr(caps), rank, n_expert,
              n_workers, _ptr(plan), _stream())
     return PeerPlan(plan, n_expert, n_workers)
@@ -579,7 +597,7 @@ def peer_plan_from_table(all_expert_count, stored_models, rank, n_expert, n_work
 def _planned_move(fn, name, buf, plan, out_rows):
     _check_cuda(buf)
     out = _recv_empty(buf, out_rows)
-    with torch.cuda.device(buf.device):
+    with _device_of(buf.device):
         _run(name, fn, _comm(buf.device), _ptr(buf), _ptr(out), _ptr(plan.buf), buf.shape[0], out_rows,
              buf.shape[1] * buf.element_size(), plan.n_expert, _stream())
     return out
@@ -601,7 +619,7 @@ def peer_scatter_planned_rows(src, row_of, row_div, scale, plan, out_rows):
         _check_cuda(scale)
         assert scale.dtype == src.dtype and scale.is_contiguous()
     out = _recv_empty(src, out_rows)
-    with torch.cuda.device(src.device):
+    with _device_of(src.device):
         _run("peer_scatter", lib.fmoe_peer_scatter_planned_rows, _comm(src.device), _ptr(src), src.shape[0], _ptr(row_of),
              int(row_div), _ptr(scale), _dtype_code(src), _ptr(out), _ptr(plan.buf), row_of.numel(), out_rows,
              src.shape[1] * src.element_size(), plan.n_expert, _stream())
@@ -621,7 +639,7 @@ def peer_scatter_fused_begin(src, row_of, row_div, scale, plan, out_rows):
         assert scale.dtype == src.dtype and scale.is_contiguous()
     out = _recv_empty(src, out_rows)
     h = _lib.Arrival()
-    with torch.cuda.device(src.device):
+    with _device_of(src.device):
         _run("peer_scatter", lib.fmoe_peer_scatter_fused_begin, _comm(src.device), _ptr(src), src.shape[0], _ptr(row_of),
              int(row_div), _ptr(scale), _dtype_code(src), _ptr(out), _ptr(plan.buf), row_of.numel(), out_rows,
              src.shape[1] * src.element_size(), plan.n_expert, _stream(), ctypes.byref(h))
@@ -642,7 +660,7 @@ class PendingArrival:
         if self.open:
             self.open = False
             dev = self.keep[0].device
-            with torch.cuda.device(dev):
+            with _device_of(dev):
                 _run("peer_arrival_finish", lib.fmoe_peer_arrival_finish, ctypes.byref(self.handle), _stream())
 
 
@@ -653,7 +671,7 @@ def peer_scatter_planned_async(input_buf, plan, out_rows, overlap_sms):
     _check_cuda(input_buf)
     out = _recv_empty(input_buf, out_rows)
     h = _lib.Arrival()
-    with torch.cuda.device(input_buf.device):
+    with _device_of(input_buf.device):
         _run("peer_scatter", lib.fmoe_peer_scatter_planned_async, _comm(input_buf.device), _ptr(input_buf), _ptr(out),
              _ptr(plan.buf), input_buf.shape[0], out_rows, input_buf.shape[1] * input_buf.element_size(), plan.n_expert,
              int(overlap_sms), _stream(), ctypes.byref(h))
@@ -667,7 +685,7 @@ def peer_gather_planned_async(output_buf, plan, out_rows, overlap_sms, use):
     _check_cuda(output_buf)
     out = _recv_empty(output_buf, out_rows)
     h = _lib.Arrival()
-    with torch.cuda.device(output_buf.device):
+    with _device_of(output_buf.device):
         _run("peer_gather", lib.fmoe_peer_gather_planned_async, _comm(output_buf.device), _ptr(output_buf), _ptr(out),
              _ptr(plan.buf), output_buf.shape[0], out_rows, output_buf.shape[1] * output_buf.element_size(),
              plan.n_expert, int(overlap_sms), int(use), _stream(), ctypes.byref(h))
@@ -685,7 +703,7 @@ def peer_gather_fused_begin(like, plan, out_rows):
     _check_cuda(like)
     out = _recv_empty(like, out_rows)
     h = _lib.Arrival()
-    with torch.cuda.device(like.device):
+    with _device_of(like.device):
         _run("peer_gather", lib.fmoe_peer_gather_fused_begin, _comm(like.device), _ptr(out), _ptr(plan.buf), out_rows,
              like.shape[1] * like.element_size(), plan.n_expert, _stream(), ctypes.byref(h))
     if not h.comm:
@@ -718,7 +736,7 @@ def exchange_cache_info(sent_models, num_expert, world_size):
     _check_cuda(sent_models)
     assert sent_models.dtype == torch.bool and sent_models.numel() == num_expert
     stored = sent_models.new_zeros((world_size, num_expert))
-    with torch.cuda.device(sent_models.device):
+    with _device_of(sent_models.device):
         _run("exchange_cache_info", lib.fmoe_exchange_cache_info, _comm(sent_models.device), _ptr(sent_models), _ptr(stored),
                                            num_expert, world_size, _stream())
     return [sent_models, stored]
@@ -734,7 +752,7 @@ def model_exchange(stored_models, local_params, params, num_expert, world_size):
     dev = local_params[0].device
     rank, world = comm_rank(dev)
     assert world == world_size
-    with torch.cuda.device(dev):
+    with _device_of(dev):
         for i in range(num_expert):
             for j in range(world_size):
                 if not flags[i + j * num_expert]:
@@ -755,7 +773,7 @@ def generate_cached_count(local_expert_count, global_expert_count, stored_models
     gec = global_expert_count.reshape(-1).to(torch.int64).contiguous()
     st = stored_models.reshape(-1).to(torch.uint8).contiguous()
     out = torch.empty_like(lec)
-    with torch.cuda.device(dev):
+    with _device_of(dev):
         _run("generate_cached_count", lib.fmoe_generate_cached_count, _ptr(lec), _ptr(gec), _ptr(st), _ptr(out), rank, num_expert,
                                              world_size, _stream())
     return out
@@ -766,7 +784,7 @@ def gradient_exchange(stored_models, local_grads, grads, num_expert, world_size)
     flags = _host_flags(stored_models)
     dev = local_grads[0].device
     rank, _ = comm_rank(dev)
-    with torch.cuda.device(dev):
+    with _device_of(dev):
         for i in range(num_expert):
             for j in range(world_size):
                 if not flags[i + j * num_expert]:
@@ -789,7 +807,7 @@ def gate_topk(logits, k):
     n_tok, n_exp = logits.shape
     val = logits.new_empty((n_tok, k))
     idx = torch.empty((n_tok, k), dtype=torch.int64, device=logits.device)
-    with torch.cuda.device(logits.device):
+    with _device_of(logits.device):
         _run("gate_topk", lib.fmoe_gate_topk, _ptr(logits), n_tok, n_exp, k, _dtype_code(logits), _ptr(val), _ptr(idx),
              _stream())
     return val, idx
@@ -801,7 +819,7 @@ def gate_topk_backward(grad_values, indices, n_expert_total):
     grad_values = grad_values.contiguous()
     n_tok, k = indices.shape
     out = grad_values.new_empty((n_tok, n_expert_total))
-    with torch.cuda.device(grad_values.device):
+    with _device_of(grad_values.device):
         _run("gate_topk_backward", lib.fmoe_gate_topk_backward, _ptr(grad_values), _ptr(indices), n_tok, n_expert_total, k,
              _dtype_code(grad_values), _ptr(out), _stream())
     return out
@@ -821,7 +839,7 @@ def count_and_pos(gate, n_expert_total, want_inv=True):
     off = torch.empty(n_expert_total + 1, dtype=torch.int64, device=dev)
     pos = torch.empty(n, dtype=torch.int64, device=dev)
     inv = torch.empty(n, dtype=torch.int64, device=dev) if want_inv else None
-    with torch.cuda.device(dev):
+    with _device_of(dev):
         scratch = _routing_scratch(n, n_expert_total, dev)
         _run("count_and_pos", lib.fmoe_count_and_pos, _ptr(gate), n, n_expert_total, _ptr(lec), _ptr(off), _ptr(pos),
                                      _ptr(inv), _ptr(scratch), _stream())
@@ -833,7 +851,7 @@ def local_scatter(inp, pos, pos_div=1, n_rows=None):
     _check_cuda(inp, pos)
     n = pos.numel() if n_rows is None else n_rows
     out = inp.new_empty((n, inp.shape[1]))
-    with torch.cuda.device(inp.device):
+    with _device_of(inp.device):
         _run("local_scatter", lib.fmoe_local_scatter, _ptr(inp), _ptr(pos), _ptr(out), n, inp.shape[0],
                                      inp.shape[1] * inp.element_size(), pos_div, _stream())
     return out
@@ -843,7 +861,7 @@ def local_gather(buf, pos, out_rows):
     """zeros(out_rows, d) with out[pos[i]] = buf[i] (index_copy_ semantics)."""
     _check_cuda(buf, pos)
     out = buf.new_empty((out_rows, buf.shape[1]))
-    with torch.cuda.device(buf.device):
+    with _device_of(buf.device):
         inv = torch.empty(out_rows, dtype=torch.int64, device=buf.device)
         _run("local_gather", lib.fmoe_local_gather, _ptr(buf), _ptr(pos), _ptr(out), pos.numel(), out_rows,
                                     buf.shape[1] * buf.element_size(), _ptr(inv), _stream())
@@ -854,7 +872,7 @@ def local_gather_inv(buf, inv):
     """out[r] = buf[inv[r]] (zero row where inv[r] < 0)."""
     _check_cuda(buf, inv)
     out = buf.new_empty((inv.numel(), buf.shape[1]))
-    with torch.cuda.device(buf.device):
+    with _device_of(buf.device):
         _run("local_gather_inv", lib.fmoe_local_gather_inv, _ptr(buf), _ptr(inv), _ptr(out), inv.numel(),
                                         buf.shape[1] * buf.element_size(), _stream())
     return out
@@ -864,7 +882,7 @@ def local_gather_sum(buf, inv, n_tokens, top_k):
     """out[t] = sum_j buf[inv[t*top_k+j]] over valid slots (deterministic index_add_)."""
     _check_cuda(buf, inv)
     out = buf.new_empty((n_tokens, buf.shape[1]))
-    with torch.cuda.device(buf.device):
+    with _device_of(buf.device):
         _run("local_gather_sum", lib.fmoe_local_gather_sum, _ptr(buf), _ptr(inv), _ptr(out), n_tokens, top_k, buf.shape[1],
                                         _dtype_code(buf), _stream())
     return out
@@ -875,7 +893,7 @@ def local_gather_add(buf, pos, out_rows):
     in ascending i (fmoe/functions.py:77-81)."""
     _check_cuda(buf, pos)
     out = buf.new_empty((out_rows, buf.shape[1]))
-    with torch.cuda.device(buf.device):
+    with _device_of(buf.device):
         scratch = _scratch(lib.fmoe_local_gather_add_scratch_bytes(out_rows), buf.device)
         _run("local_gather_add", lib.fmoe_local_gather_add, _ptr(buf), _ptr(pos), _ptr(out), pos.numel(), out_rows,
              buf.shape[1], _dtype_code(buf), _ptr(scratch), _stream())
@@ -888,7 +906,7 @@ def combine_forward(buf, inv, score):
     n_tokens, top_k = score.shape
     assert score.dtype == buf.dtype
     out = buf.new_empty((n_tokens, buf.shape[1]))
-    with torch.cuda.device(buf.device):
+    with _device_of(buf.device):
         _run("combine_forward", lib.fmoe_combine_forward, _ptr(buf), _ptr(inv), _ptr(score), _ptr(out), n_tokens, top_k,
                                        buf.shape[1], _dtype_code(buf), _stream())
     return out
@@ -903,7 +921,7 @@ def combine_backward(grad_out, buf, inv, score, need_score_grad=True, need_buf_g
         return None, None
     grad_buf = torch.empty_like(buf) if need_buf_grad else None
     grad_score = torch.empty_like(score) if need_score_grad else None
-    with torch.cuda.device(buf.device):
+    with _device_of(buf.device):
         _run("combine_backward", lib.fmoe_combine_backward, _ptr(grad_out), _ptr(buf), _ptr(inv), _ptr(score), _ptr(grad_buf),
                                         _ptr(grad_score), n_tokens, top_k, buf.shape[1], _dtype_code(buf),
                                         _stream())
@@ -924,7 +942,7 @@ def linear_forward_act(x, seg_offsets, weight, bias, activation, want_pre=False,
     y = out if out is not None else x.new_empty((x.shape[0], out_feat))
     assert y.shape == (x.shape[0], out_feat) and y.dtype == x.dtype and y.is_contiguous()
     pre = x.new_empty((x.shape[0], out_feat)) if want_pre else None
-    with torch.cuda.device(x.device):
+    with _device_of(x.device):
         arriving = arrival is not None and arrival.open
         if arriving or departure is not None:
             if arriving:
@@ -954,7 +972,7 @@ def linear_backward_act(grad_y, x, seg_offsets, weight, act_pre, activation, nee
     gx = (grad_x if grad_x is not None else x.new_empty((n_rows, in_feat))) if need_input_grad else None
     gw = grad_w if grad_w is not None else torch.empty_like(weight)
     gb = grad_b if grad_b is not None else (weight.new_empty((n_expert, out_feat)) if need_bias else None)
-    with torch.cuda.device(x.device):
+    with _device_of(x.device):
         nbytes = lib.fmoe_linear_scratch_bytes(n_rows, in_feat, out_feat, n_expert, _dtype_code(x))
         scratch = _scratch(nbytes, x.device)
         arriving = arrival is not None and arrival.open
@@ -981,6 +999,65 @@ def linear_backward_act(grad_y, x, seg_offsets, weight, act_pre, activation, nee
                                        out_feat, n_expert, _dtype_code(x), activation,
                                        1 if accumulate else 0, _ptr(scratch), _stream())
     return gx, gw, gb
+
+
+# ---------------------------------------------------------------------------
+# One layer call on one GPU (bucketing, scatter, experts, gather) in one library call each way
+# ---------------------------------------------------------------------------
+
+@functools.lru_cache(maxsize=256)
+def _moe_mlp_bytes(*sizes):
+    args = _lib.MoeMlp(*(None,) * 18, *sizes, 0)
+    out = [ctypes.c_int64() for _ in range(3)]
+    check(lib.fmoe_moe_mlp_bytes(ctypes.byref(args), *(ctypes.byref(v) for v in out)), "moe_mlp_bytes")
+    return tuple(v.value for v in out)
+
+
+class MoeMlpCall:
+    """Sizes and buffers of one layer call, kept from its forward to its backward (without tensors)."""
+    __slots__ = ("sizes", "n_bytes", "bias")
+
+    def __init__(self, n_tokens, top_k, w1, activation, keep, bias):
+        n_expert, d_hidden, d_model = w1.shape
+        self.sizes = (n_tokens, d_model, d_hidden, top_k, n_expert, _DT[w1.dtype], activation, 1 if keep else 0)
+        self.n_bytes = _moe_mlp_bytes(*self.sizes)
+        self.bias = bias
+
+
+def moe_mlp_forward(call, inp, gate_idx, score, w1, b1, w2, b2):
+    """Returns (out, index, rows); the last two are what moe_mlp_backward reads (call.sizes[-1] set)."""
+    _check_cuda(inp, gate_idx, score, w1, b1, w2, b2)
+    dev = inp.device
+    out = torch.empty_like(inp)
+    index = torch.empty(call.n_bytes[0], dtype=torch.uint8, device=dev)
+    rows = torch.empty(call.n_bytes[1], dtype=torch.uint8, device=dev)
+    args = _lib.MoeMlp(inp.data_ptr(), gate_idx.data_ptr(), score.data_ptr(), w1.data_ptr(),
+                       None if b1 is None else b1.data_ptr(), w2.data_ptr(), None if b2 is None else b2.data_ptr(),
+                       index.data_ptr(), rows.data_ptr(), out.data_ptr(), *(None,) * 8, *call.sizes, 0)
+    with _device_of(dev):
+        check(lib.fmoe_moe_mlp_forward(ctypes.byref(args), _stream()), "moe_mlp_forward")
+    return out, index, rows
+
+
+def moe_mlp_backward(call, grad_out, score, w1, w2, index, rows, need_experts, need_input, need_score):
+    """Returns (grad_inp, grad_score, gw1, gb1, gw2, gb2), None where not asked for."""
+    _check_cuda(grad_out, score, w1, w2)
+    dev = grad_out.device
+    need_experts = need_experts or need_input
+    gscore = torch.empty_like(score) if need_score else None
+    ginp = torch.empty_like(grad_out) if need_input else None
+    grads = gw1 = gb1 = gw2 = gb2 = None
+    if need_experts:
+        grads = torch.empty(call.n_bytes[2], dtype=torch.uint8, device=dev)
+        gw1, gw2 = torch.empty_like(w1), torch.empty_like(w2)
+        gb1 = w1.new_empty((w1.shape[0], w1.shape[1])) if call.bias[0] else None
+        gb2 = w2.new_empty((w2.shape[0], w2.shape[1])) if call.bias[1] else None
+    ptr = [None if t is None else t.data_ptr() for t in (grads, ginp, gscore, gw1, gb1, gw2, gb2)]
+    args = _lib.MoeMlp(None, None, score.data_ptr(), w1.data_ptr(), None, w2.data_ptr(), None, index.data_ptr(),
+                       rows.data_ptr(), None, grad_out.data_ptr(), *ptr, *call.sizes, 0)
+    with _device_of(dev):
+        check(lib.fmoe_moe_mlp_backward(ctypes.byref(args), _stream()), "moe_mlp_backward")
+    return ginp, gscore, gw1, gb1, gw2, gb2
 
 
 # ---------------------------------------------------------------------------
@@ -1086,7 +1163,7 @@ def fused_forward(input_buf, params, local_expert_count, global_expert_count, st
     gob = input_buf.new_empty((B + S, d_model))
     out = input_buf.new_empty((A, d_model))
     table, keep = _mlp_table(params, None, n_workers)
-    with torch.cuda.device(dev):
+    with _device_of(dev):
         comm = _comm(dev) if n_workers > 1 else None
         _run("fused_forward", lib.fmoe_fused_forward, comm, _ptr(input_buf), _ptr(out), _ptr(gib), _ptr(gmb),
              _ptr(pre), _ptr(gob), table, _ptr(lec), _ptr(gec), _ptr(st), A, d_model, d_hidden, n_expert,
@@ -1134,7 +1211,7 @@ def fused_backward(input_buf, params, middle_buf, output_buf, grad_out, local_ex
     grad_in = input_buf.new_empty((grad_out.shape[0], d_model))
     table, keep = _mlp_table(params, grads, n_workers)
     gran = fuse_gran()
-    with torch.cuda.device(dev):
+    with _device_of(dev):
         comm = _comm(dev) if n_workers > 1 else None
         _run("fused_backward", lib.fmoe_fused_backward, comm, _ptr(grad_out), _ptr(grad_in), _ptr(input_buf),
              _ptr(middle_buf), _ptr(middle_pre), _ptr(ggo), _ptr(gmid), _ptr(ggi), table, _ptr(lec), _ptr(gec),

@@ -568,11 +568,11 @@ class FusedExpertMLP(Function):
     applied in the epilogue of the second layer's input-gradient GEMM."""
 
     @staticmethod
-    def forward(ctx, x, offsets, w1, b1, w2, b2, act, exch=None):
-        """``exch``: the PlannedExchange whose scatter produced ``x`` (and whose scatter of the output
+    def forward(ctx, x, offsets, w1, b1, w2, b2, act, exch=None, keep=True):
+        """``keep``: a backward may follow.  ``exch``: the PlannedExchange whose scatter produced ``x`` (and whose scatter of the output
         gradient will produce ``grad_y``); a pending arrival of it is waited for tile by tile."""
         x = x.contiguous()
-        want_pre = act == _lib.ACT_GELU and (x.requires_grad or w1.requires_grad)
+        want_pre = keep and act == _lib.ACT_GELU and (x.requires_grad or w1.requires_grad)
         arrival = exch.take_pending() if exch is not None else None
         h, pre = fmoe_cuda.linear_forward_act(x, offsets, w1, b1, act, want_pre=want_pre, arrival=arrival)
         y = x.new_empty((x.shape[0], w2.shape[1]))
@@ -611,7 +611,35 @@ class FusedExpertMLP(Function):
         gx, gw1, _ = fmoe_cuda.linear_backward_act(gh, x, offsets, w1, None, _lib.ACT_NONE, need_bias=False,
                                                    need_input_grad=ctx.needs_input_grad[0], departure=departure,
                                                    grad_x=gx)
-        return gx, None, gw1, gb1, gw2, gb2, None, None
+        return gx, None, gw1, gb1, gw2, gb2, None, None, None
+
+
+class MoeMlp(Function):
+    """Everything between the gate and the layer's output on one GPU -- bucketing, scatter, FusedExpertMLP, gather and
+    combine -- in one library call each way: the same kernels as MOEScatterFused, FusedExpertMLP and MOEGatherCombine
+    in the same order, without the host work between them."""
+
+    @staticmethod
+    def forward(ctx, inp, gate_idx, score, w1, b1, w2, b2, act, keep):
+        """``keep``: a backward may follow (False: nothing is stored for one)."""
+        inp = inp.contiguous()
+        score_c = score.contiguous().to(inp.dtype)
+        call = fmoe_cuda.MoeMlpCall(gate_idx.shape[0], gate_idx.shape[1], w1, act, keep, (b1 is not None, b2 is not None))
+        out, index, rows = fmoe_cuda.moe_mlp_forward(call, inp, gate_idx, score_c, w1, b1, w2, b2)
+        if keep:
+            ctx.call, ctx.score_dtype = call, score.dtype
+            ctx.save_for_backward(score_c, w1, w2, index, rows)
+        return out
+
+    @staticmethod
+    def backward(ctx, grad_out):
+        score, w1, w2, index, rows = ctx.saved_tensors
+        need = ctx.needs_input_grad
+        ginp, gscore, gw1, gb1, gw2, gb2 = fmoe_cuda.moe_mlp_backward(
+            ctx.call, grad_out.contiguous(), score, w1, w2, index, rows, any(need[3:7]), need[0], need[2])
+        if gscore is not None:
+            gscore = gscore.to(ctx.score_dtype)
+        return ginp, None, gscore, gw1, gb1, gw2, gb2, None, None
 
 
 class AllGather(Function):

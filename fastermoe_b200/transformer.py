@@ -17,6 +17,9 @@ POLICY_CONSTANTS = {
 }
 
 
+_KERNEL_DTYPES = (torch.float32, torch.float16, torch.bfloat16)
+
+
 class _Expert(nn.Module):
     r"""All experts of one worker as two grouped linear layers with an activation
     in between (fmoe/transformer.py:10-30).  When the activation is ReLU or
@@ -33,6 +36,23 @@ class _Expert(nn.Module):
         exchange that are still arriving (and later on the arriving output gradient)."""
         return inp.is_cuda and activation_code(self.activation) is not None
 
+    def whole_layer_operands(self, inp):
+        """(activation code, w1, b1, w2, b2) when nothing can tell a call of forward() from the fused layer call on
+        the same parameters; else None."""
+        if (type(self) is not _Expert or "forward" in self.__dict__ or self._forward_hooks or self._forward_pre_hooks or
+                self._backward_hooks or self._backward_pre_hooks or self._compiled_call_impl is not None or
+                torch.nn.modules.module._has_any_global_hook()):
+            return None
+        code = activation_code(self.activation)
+        up, down = self.htoh4, self.h4toh
+        w1, b1, w2, b2 = up.weight, up.bias, down.weight, down.bias
+        if code is None or inp.dtype not in _KERNEL_DTYPES or inp.dim() != 2 or inp.shape[1] != w1.shape[2]:
+            return None
+        for t in (w1, b1, w2, b2):
+            if t is not None and (t.dtype != inp.dtype or t.device != inp.device or not t.is_contiguous()):
+                return None
+        return code, w1, b1, w2, b2
+
     def forward(self, inp, fwd_expert_count):
         code = activation_code(self.activation)
         exch = getattr(fwd_expert_count, "exchange", None)
@@ -44,7 +64,7 @@ class _Expert(nn.Module):
             return self.h4toh(x, fwd_expert_count)
         counts = ExpertCounts.wrap(fwd_expert_count, inp.device)
         return FusedExpertMLP.apply(inp, counts.offsets, self.htoh4.weight, self.htoh4.bias,
-                                    self.h4toh.weight, self.h4toh.bias, code, exch)
+                                    self.h4toh.weight, self.h4toh.bias, code, exch, torch.is_grad_enabled())
 
 
 def _gen_policy(alpha, constants=None):

@@ -692,6 +692,55 @@ int fmoe_fused_backward(fmoe_comm_t comm, const void* grad_out_local, void* grad
                         int32_t pipeline_gran, void* staging, fmoe_stream_t stream,
                         fmoe_stream_t comm_stream);
 
+/* ------------------------------------------------------------------------
+ * One MoE MLP layer call on one GPU as one host call: bucketing of the gate
+ * entries, local scatter, both expert products with the activation between
+ * them, and the score-weighted gather.  Device work, order and results are
+ * those of the single operators above.
+ *   forward : gate_idx [n_tokens, top_k], inp, score (dtype of inp), w1/b1/w2/b2
+ *             (biases may be NULL) -> out; index and rows are buffers of
+ *             fmoe_moe_mlp_bytes, whose contents the backward needs when
+ *             keep != 0.  They may be discarded after a forward with keep == 0.
+ *   backward: score, w1, w2, index, rows as the forward saw or left them,
+ *             grad_out -> grad_score (or NULL), and, unless gw1 is NULL,
+ *             gw1, gw2, gb1 and gb2 (NULL without biases) and grad_inp (or
+ *             NULL); grads is a scratch buffer of fmoe_moe_mlp_bytes.
+ * All buffers 16-byte aligned; n_tokens > 0.
+ * ---------------------------------------------------------------------- */
+typedef struct {
+    const void* inp;
+    const int64_t* gate_idx;
+    const void* score;
+    const void* w1;
+    const void* b1;
+    const void* w2;
+    const void* b2;
+    void* index;
+    void* rows;
+    void* out;
+    const void* grad_out;
+    void* grads;
+    void* grad_inp;
+    void* grad_score;
+    void* gw1;
+    void* gb1;
+    void* gw2;
+    void* gb2;
+    int64_t n_tokens;
+    int64_t d_model;
+    int64_t d_hidden;
+    int32_t top_k;
+    int32_t n_expert;
+    int32_t dtype;
+    int32_t activation;
+    int32_t keep;
+    int32_t reserved;
+} fmoe_moe_mlp_t;
+
+int fmoe_moe_mlp_bytes(const fmoe_moe_mlp_t* args, int64_t* index_bytes, int64_t* row_bytes, int64_t* grad_bytes);
+int fmoe_moe_mlp_forward(const fmoe_moe_mlp_t* args, fmoe_stream_t stream);
+int fmoe_moe_mlp_backward(const fmoe_moe_mlp_t* args, fmoe_stream_t stream);
+
 #ifdef __cplusplus
 }
 #endif

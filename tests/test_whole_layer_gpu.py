@@ -1,0 +1,88 @@
+"""The layer as one library call against the same layer operator by operator, and the calls that must not take it."""
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+ACTS = {"gelu": torch.nn.GELU, "relu": torch.nn.ReLU}
+
+
+def make(T, d, h, E, k, act="gelu", dtype=torch.bfloat16, bias=True, softmax=True, seed=0):
+    from fastermoe_b200 import FMoETransformerMLP
+    torch.manual_seed(seed)
+    m = FMoETransformerMLP(num_expert=E, d_model=d, d_hidden=h, top_k=k, activation=ACTS[act](), bias=bias)
+    for p in m.parameters():
+        torch.nn.init.uniform_(p, -d ** -0.5, d ** -0.5)
+    m.gate.softmax_scores = softmax
+    x = torch.randn(T, d, device="cuda").to(dtype).requires_grad_(True)
+    return m.cuda().to(dtype), x
+
+
+def step(m, x, g):
+    x.grad = None
+    m.zero_grad()
+    out = m(x)
+    out.backward(g)
+    return [out.detach(), x.grad] + [p.grad for p in m.parameters()]
+
+
+@pytest.mark.parametrize("act", list(ACTS))
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("T,d,h,E,k,bias", [(1, 256, 512, 4, 2, True), (67, 256, 512, 8, 2, False), (130, 72, 200, 5, 3, True),
+                                            (33, 30, 50, 3, 1, True), (700, 264, 136, 40, 8, False)])
+def test_one_call_equals_the_operators(act, dtype, T, d, h, E, k, bias):
+    """Same kernels in the same order: equal to the last bit, and every output is written."""
+    m, x = make(T, d, h, E, k, act, dtype, bias)
+    g = torch.randn(T, d, device="cuda").to(dtype)
+    from fastermoe_b200 import fmoe_cuda as fc
+    one = step(m, x, g)
+    fc.set_profile(fc.Profile())            # operator by operator
+    try:
+        parts = step(m, x, g)
+    finally:
+        fc.set_profile(None)
+    for a, b in zip(one, parts):
+        assert torch.equal(a, b)
+    with torch.no_grad():
+        assert torch.equal(m(x), one[0])
+    assert m(x.detach()).shape == x.shape and all(torch.isfinite(t.float()).all() for t in one)
+
+
+def test_partial_gradients():
+    """Only what requires a gradient gets one."""
+    m, x = make(50, 256, 512, 4, 2)
+    g = torch.randn(50, 256, device="cuda").bfloat16()
+    want = step(m, x, g)
+    m.experts.requires_grad_(False)
+    got = step(m, x, g)
+    assert torch.equal(got[1], want[1]) and m.experts.htoh4.weight.grad is None
+    assert torch.equal(m.gate.gate.weight.grad, want[2 + [n for n, _ in m.named_parameters()].index("gate.gate.weight")])
+    m.experts.requires_grad_(True)
+    m(x.detach()).backward(g)
+    for (n, p), w in zip(m.named_parameters(), want[2:]):
+        torch.testing.assert_close(p.grad, w if n.startswith("gate") else p.grad)
+    m.zero_grad()
+    m.requires_grad_(False)
+    x.grad = None
+    m(x).backward(g)
+    assert torch.equal(x.grad, want[1])
+
+
+@pytest.mark.parametrize("act", ["gelu"])
+def test_hooks_are_called(act):
+    m, x = make(20, 256, 512, 4, 2, act)
+    base = m(x)
+    seen = []
+    hooks = [m.experts.register_forward_hook(lambda *a: seen.append("experts"))]
+    if act == "silu":       # the two linears and the activation are calls of their own then
+        hooks += [getattr(m.experts, n).register_forward_hook(lambda *a, n=n: seen.append(n)) for n in ("htoh4", "activation")]
+    out = m(x)
+    assert seen == (["htoh4", "activation", "experts"] if act == "silu" else ["experts"])
+    torch.testing.assert_close(out, base, rtol=2e-2, atol=2e-2)
+    for h in hooks:
+        h.remove()
+    out = m.experts_out = []
+    m.expert_fn, plain = (lambda inp, *a: (out.append(inp.shape), plain(inp, *a))[1]), m.expert_fn
+    m(x)
+    assert out == [(40, 256)]
