@@ -25,7 +25,21 @@ __device__ __forceinline__ bool ranks_before(float a, int ia, float b, int ib) {
     return ia < ib;
 }
 
+// Softmax over the k selected logits (best[0] is the largest; NaN ranks first), as values of T.
 template <typename T>
+__device__ __forceinline__ void store_softmax(const float (&best)[kTopKMax], int k, T* __restrict__ values) {
+    float p[kTopKMax], sum = 0.f;
+#pragma unroll
+    for (int j = 0; j < kTopKMax; ++j)
+        if (j < k) { p[j] = expf(best[j] - best[0]); sum += p[j]; }
+#pragma unroll
+    for (int j = 0; j < kTopKMax; ++j)
+        if (j < k) values[j] = from_float<T>(p[j] / sum);
+}
+
+// SOFTMAX: the values are the softmax over the selected logits.  As an operator of its own that softmax cost a launch
+// in each direction (1.4-2 us of device time, 10 us of host time) for k values per token.
+template <typename T, bool SOFTMAX>
 __global__ void __launch_bounds__(256)
 topk_forward_kernel(const T* __restrict__ logits, int64_t n_tokens, int n_expert, int k, T* __restrict__ values,
                     int64_t* __restrict__ indices) {
@@ -50,7 +64,10 @@ topk_forward_kernel(const T* __restrict__ logits, int64_t n_tokens, int n_expert
             }
         }
     }
-    for (int j = 0; j < k; ++j) {
+    float won[kTopKMax];
+#pragma unroll
+    for (int j = 0; j < kTopKMax; ++j) {
+        if (j >= k) break;
         float v = best[0];
         int vi = best_i[0];
 #pragma unroll
@@ -64,16 +81,18 @@ topk_forward_kernel(const T* __restrict__ logits, int64_t n_tokens, int n_expert
             for (int q = 0; q + 1 < kTopKMax; ++q) { best[q] = best[q + 1]; best_i[q] = best_i[q + 1]; }
             best[kTopKMax - 1] = -INFINITY; best_i[kTopKMax - 1] = INT_MAX;
         }
+        won[j] = v;
         if (lane == 0) {
-            values[tok * k + j] = row[vi];
+            if (!SOFTMAX) values[tok * k + j] = row[vi];
             indices[tok * k + j] = vi;
         }
     }
+    if (SOFTMAX && lane == 0) store_softmax<T>(won, k, values + tok * k);
 }
 
 // Few experts (<= 32): one THREAD per token; a warp then reads 32 consecutive rows, i.e. one
 // contiguous stretch of the logits, and no lane idles.  Same order as the warp kernel.
-template <typename T>
+template <typename T, bool SOFTMAX>
 __global__ void __launch_bounds__(256)
 topk_forward_small_kernel(const T* __restrict__ logits, int64_t n_tokens, int n_expert, int k, T* __restrict__ values,
                           int64_t* __restrict__ indices) {
@@ -99,24 +118,29 @@ topk_forward_small_kernel(const T* __restrict__ logits, int64_t n_tokens, int n_
 #pragma unroll
     for (int j = 0; j < kTopKMax; ++j) {
         if (j < k) {
-            values[tok * k + j] = row[best_i[j]];
+            if (!SOFTMAX) values[tok * k + j] = row[best_i[j]];
             indices[tok * k + j] = best_i[j];
         }
     }
+    if (SOFTMAX) store_softmax<T>(best, k, values + tok * k);
 }
 
-template <typename T>
+template <typename T, bool SOFTMAX>
 __global__ void __launch_bounds__(256)
-topk_backward_kernel(const T* __restrict__ grad_values, const int64_t* __restrict__ indices, int64_t n_tokens,
+topk_backward_kernel(const T* __restrict__ grad_values, const T* __restrict__ probs, const int64_t* __restrict__ indices, int64_t n_tokens,
                      int n_expert, int k, T* __restrict__ grad_logits) {
     const int64_t total = n_tokens * n_expert;
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
         const int64_t tok = i / n_expert;
         const int e = (int)(i - tok * n_expert);
-        float g = 0.f;
-        for (int j = 0; j < k; ++j)
-            if (indices[tok * k + j] == e) g += to_float(grad_values[tok * k + j]);
-        grad_logits[i] = from_float<T>(g);
+        float g = 0.f, p = 0.f, dot = 0.f;
+        for (int j = 0; j < k; ++j) {
+            const float gj = to_float(grad_values[tok * k + j]);
+            const float pj = SOFTMAX ? to_float(probs[tok * k + j]) : 1.f;
+            if (SOFTMAX) dot = fmaf(pj, gj, dot);
+            if (indices[tok * k + j] == e) { g += pj * gj; p += pj; }
+        }
+        grad_logits[i] = from_float<T>(SOFTMAX && p != 0.f ? g - p * dot : g);
     }
 }
 
@@ -125,49 +149,71 @@ topk_backward_kernel(const T* __restrict__ grad_values, const int64_t* __restric
 
 using namespace fmoe;
 
-extern "C" int fmoe_gate_topk(const void* logits, int64_t n_tokens, int32_t n_expert_total, int32_t k, int32_t dtype,
-                              void* values, int64_t* indices, fmoe_stream_t stream) {
+namespace {
+
+template <typename T, bool SOFTMAX>
+void launch_topk(const void* logits, int64_t n_tokens, int n_expert, int k, void* values, int64_t* indices, cudaStream_t st) {
+    if (n_expert <= 32)
+        topk_forward_small_kernel<T, SOFTMAX><<<(unsigned)ceil_div(n_tokens, 256), 256, 0, st>>>((const T*)logits, n_tokens, n_expert, k, (T*)values, indices);
+    else
+        topk_forward_kernel<T, SOFTMAX><<<(unsigned)ceil_div(n_tokens, 8), 256, 0, st>>>((const T*)logits, n_tokens, n_expert, k, (T*)values, indices);
+}
+
+template <bool SOFTMAX>
+int topk(const void* logits, int64_t n_tokens, int32_t n_expert_total, int32_t k, int32_t dtype, void* values, int64_t* indices,
+         cudaStream_t st) {
     FMOE_REQUIRE(n_tokens >= 0 && n_expert_total > 0, "gate_topk: n_tokens=%lld n_expert_total=%d", (long long)n_tokens,
                  n_expert_total);
     FMOE_REQUIRE(k >= 1 && k <= kTopKMax && k <= n_expert_total, "gate_topk: k=%d (1..%d, <= n_expert_total)", k, kTopKMax);
     FMOE_REQUIRE(dtype_size(dtype) > 0, "gate_topk: unknown dtype %d", dtype);
     if (n_tokens == 0) return 0;
     FMOE_REQUIRE(logits && values && indices, "gate_topk: null pointer");
-    cudaStream_t st = (cudaStream_t)stream;
-    if (n_expert_total <= 32) {
-        const unsigned nb = (unsigned)ceil_div(n_tokens, 256);
-        switch (dtype) {
-            case FMOE_F32: topk_forward_small_kernel<float><<<nb, 256, 0, st>>>((const float*)logits, n_tokens, n_expert_total, k, (float*)values, indices); break;
-            case FMOE_F16: topk_forward_small_kernel<__half><<<nb, 256, 0, st>>>((const __half*)logits, n_tokens, n_expert_total, k, (__half*)values, indices); break;
-            default: topk_forward_small_kernel<__nv_bfloat16><<<nb, 256, 0, st>>>((const __nv_bfloat16*)logits, n_tokens, n_expert_total, k, (__nv_bfloat16*)values, indices); break;
-        }
-        FMOE_CHECK_LAUNCH();
-        return 0;
-    }
-    const unsigned blocks = (unsigned)ceil_div(n_tokens, 8);
     switch (dtype) {
-        case FMOE_F32: topk_forward_kernel<float><<<blocks, 256, 0, st>>>((const float*)logits, n_tokens, n_expert_total, k, (float*)values, indices); break;
-        case FMOE_F16: topk_forward_kernel<__half><<<blocks, 256, 0, st>>>((const __half*)logits, n_tokens, n_expert_total, k, (__half*)values, indices); break;
-        default: topk_forward_kernel<__nv_bfloat16><<<blocks, 256, 0, st>>>((const __nv_bfloat16*)logits, n_tokens, n_expert_total, k, (__nv_bfloat16*)values, indices); break;
+        case FMOE_F32: launch_topk<float, SOFTMAX>(logits, n_tokens, n_expert_total, k, values, indices, st); break;
+        case FMOE_F16: launch_topk<__half, SOFTMAX>(logits, n_tokens, n_expert_total, k, values, indices, st); break;
+        default: launch_topk<__nv_bfloat16, SOFTMAX>(logits, n_tokens, n_expert_total, k, values, indices, st); break;
     }
     FMOE_CHECK_LAUNCH();
     return 0;
 }
 
-extern "C" int fmoe_gate_topk_backward(const void* grad_values, const int64_t* indices, int64_t n_tokens,
-                                       int32_t n_expert_total, int32_t k, int32_t dtype, void* grad_logits,
-                                       fmoe_stream_t stream) {
+template <bool SOFTMAX>
+int topk_backward(const void* grad, const void* probs, const int64_t* indices, int64_t n_tokens, int32_t n_expert_total, int32_t k,
+                  int32_t dtype, void* grad_logits, cudaStream_t st) {
     FMOE_REQUIRE(n_tokens >= 0 && n_expert_total > 0 && k >= 1 && k <= kTopKMax, "gate_topk_backward: bad sizes");
     FMOE_REQUIRE(dtype_size(dtype) > 0, "gate_topk_backward: unknown dtype %d", dtype);
     if (n_tokens == 0) return 0;
-    FMOE_REQUIRE(grad_values && indices && grad_logits, "gate_topk_backward: null pointer");
-    cudaStream_t st = (cudaStream_t)stream;
+    FMOE_REQUIRE(grad && indices && grad_logits && (!SOFTMAX || probs), "gate_topk_backward: null pointer");
     const unsigned blocks = (unsigned)std::min<int64_t>(ceil_div(n_tokens * n_expert_total, 256), 148 * 16);
     switch (dtype) {
-        case FMOE_F32: topk_backward_kernel<float><<<blocks, 256, 0, st>>>((const float*)grad_values, indices, n_tokens, n_expert_total, k, (float*)grad_logits); break;
-        case FMOE_F16: topk_backward_kernel<__half><<<blocks, 256, 0, st>>>((const __half*)grad_values, indices, n_tokens, n_expert_total, k, (__half*)grad_logits); break;
-        default: topk_backward_kernel<__nv_bfloat16><<<blocks, 256, 0, st>>>((const __nv_bfloat16*)grad_values, indices, n_tokens, n_expert_total, k, (__nv_bfloat16*)grad_logits); break;
+        case FMOE_F32: topk_backward_kernel<float, SOFTMAX><<<blocks, 256, 0, st>>>((const float*)grad, (const float*)probs, indices, n_tokens, n_expert_total, k, (float*)grad_logits); break;
+        case FMOE_F16: topk_backward_kernel<__half, SOFTMAX><<<blocks, 256, 0, st>>>((const __half*)grad, (const __half*)probs, indices, n_tokens, n_expert_total, k, (__half*)grad_logits); break;
+        default: topk_backward_kernel<__nv_bfloat16, SOFTMAX><<<blocks, 256, 0, st>>>((const __nv_bfloat16*)grad, (const __nv_bfloat16*)probs, indices, n_tokens, n_expert_total, k, (__nv_bfloat16*)grad_logits); break;
     }
     FMOE_CHECK_LAUNCH();
     return 0;
+}
+
+}  // namespace
+
+extern "C" int fmoe_gate_topk(const void* logits, int64_t n_tokens, int32_t n_expert_total, int32_t k, int32_t dtype,
+                              void* values, int64_t* indices, fmoe_stream_t stream) {
+    return topk<false>(logits, n_tokens, n_expert_total, k, dtype, values, indices, (cudaStream_t)stream);
+}
+
+extern "C" int fmoe_gate_topk_softmax(const void* logits, int64_t n_tokens, int32_t n_expert_total, int32_t k, int32_t dtype,
+                                      void* probs, int64_t* indices, fmoe_stream_t stream) {
+    return topk<true>(logits, n_tokens, n_expert_total, k, dtype, probs, indices, (cudaStream_t)stream);
+}
+
+extern "C" int fmoe_gate_topk_backward(const void* grad_values, const int64_t* indices, int64_t n_tokens,
+                                       int32_t n_expert_total, int32_t k, int32_t dtype, void* grad_logits,
+                                       fmoe_stream_t stream) {
+    return topk_backward<false>(grad_values, nullptr, indices, n_tokens, n_expert_total, k, dtype, grad_logits, (cudaStream_t)stream);
+}
+
+extern "C" int fmoe_gate_topk_softmax_backward(const void* grad_probs, const void* probs, const int64_t* indices,
+                                               int64_t n_tokens, int32_t n_expert_total, int32_t k, int32_t dtype,
+                                               void* grad_logits, fmoe_stream_t stream) {
+    return topk_backward<true>(grad_probs, probs, indices, n_tokens, n_expert_total, k, dtype, grad_logits, (cudaStream_t)stream);
 }

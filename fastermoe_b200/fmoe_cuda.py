@@ -799,29 +799,37 @@ def gradient_exchange(stored_models, local_grads, grads, num_expert, world_size)
 # Extended operators (no counterpart in the reference's extension)
 # ---------------------------------------------------------------------------
 
-def gate_topk(logits, k):
+def gate_topk(logits, k, softmax=False):
     """(values [T,k], indices [T,k] int64): the k largest logits per row (torch.topk, largest=True), in
-    descending order, ties by ascending index (fmoe/gates/naive_gate.py:31-34)."""
+    descending order, ties by ascending index (fmoe/gates/naive_gate.py:31-34).  ``softmax``: the values are
+    the softmax over the k selected logits (computed in fp32)."""
     _check_cuda(logits)
     logits = logits.contiguous()
     n_tok, n_exp = logits.shape
     val = logits.new_empty((n_tok, k))
     idx = torch.empty((n_tok, k), dtype=torch.int64, device=logits.device)
     with _device_of(logits.device):
-        _run("gate_topk", lib.fmoe_gate_topk, _ptr(logits), n_tok, n_exp, k, _dtype_code(logits), _ptr(val), _ptr(idx),
-             _stream())
+        _run("gate_topk", lib.fmoe_gate_topk_softmax if softmax else lib.fmoe_gate_topk, _ptr(logits), n_tok, n_exp, k,
+             _dtype_code(logits), _ptr(val), _ptr(idx), _stream())
     return val, idx
 
 
-def gate_topk_backward(grad_values, indices, n_expert_total):
-    """Gradient of gate_topk with respect to the logits ([T, n_expert_total])."""
-    _check_cuda(grad_values, indices)
+def gate_topk_backward(grad_values, indices, n_expert_total, probs=None):
+    """Gradient of gate_topk with respect to the logits ([T, n_expert_total]); ``probs``: the values of the
+    softmax form."""
+    _check_cuda(indices, probs)
+    if not grad_values.is_cuda:
+        raise RuntimeError("fmoe_cuda: expected a CUDA tensor")
     grad_values = grad_values.contiguous()
     n_tok, k = indices.shape
     out = grad_values.new_empty((n_tok, n_expert_total))
     with _device_of(grad_values.device):
-        _run("gate_topk_backward", lib.fmoe_gate_topk_backward, _ptr(grad_values), _ptr(indices), n_tok, n_expert_total, k,
-             _dtype_code(grad_values), _ptr(out), _stream())
+        if probs is not None:
+            _run("gate_topk_backward", lib.fmoe_gate_topk_softmax_backward, _ptr(grad_values), _ptr(probs), _ptr(indices),
+                 n_tok, n_expert_total, k, _dtype_code(grad_values), _ptr(out), _stream())
+        else:
+            _run("gate_topk_backward", lib.fmoe_gate_topk_backward, _ptr(grad_values), _ptr(indices), n_tok, n_expert_total,
+                 k, _dtype_code(grad_values), _ptr(out), _stream())
     return out
 
 

@@ -660,33 +660,44 @@ class AllGather(Function):
 
 class GateTopK(Function):
     """torch.topk(logits, k, largest=True) on the last dimension of a 2-D CUDA tensor with the
-    library's kernels (fmoe/gates/naive_gate.py:31-34): returns (values, indices), descending."""
+    library's kernels (fmoe/gates/naive_gate.py:31-34): returns (values, indices), descending; with ``softmax`` the
+    values are the softmax over the k selected logits, formed in the same kernel."""
 
     @staticmethod
-    def forward(ctx, logits, k):
-        val, idx = fmoe_cuda.gate_topk(logits, k)
-        ctx.n_expert = logits.shape[1]
-        ctx.save_for_backward(idx)
+    def forward(ctx, logits, k, softmax=False):
+        val, idx = fmoe_cuda.gate_topk(logits, k, softmax)
+        ctx.n_expert, ctx.softmax = logits.shape[1], softmax
+        if softmax:
+            ctx.save_for_backward(idx, val)
+        else:
+            ctx.save_for_backward(idx)
         ctx.mark_non_differentiable(idx)
+        ctx.set_materialize_grads(False)        # (the indices would get a gradient of zeros on every backward)
         return val, idx
 
     @staticmethod
     def backward(ctx, grad_val, _grad_idx):
-        (idx,) = ctx.saved_tensors
-        return fmoe_cuda.gate_topk_backward(grad_val, idx, ctx.n_expert), None
+        if grad_val is None:
+            return None, None, None
+        idx, *probs = ctx.saved_tensors
+        return fmoe_cuda.gate_topk_backward(grad_val, idx, ctx.n_expert, *probs), None, None
 
 
-def gate_topk(logits, k):
+def gate_topk(logits, k, softmax=False):
     """Top-k over the last dimension with the library's kernel (CUDA tensors; k <= 8).  A CPU
-    tensor, which no GPU code path produces, is answered by torch.topk.  Returns (values, indices)."""
+    tensor, which no GPU code path produces, is answered by torch.topk.  Returns (values, indices);
+    ``softmax``: the values are the softmax over the selected logits."""
     if logits.is_cuda:
         if k > 8 or logits.dtype not in (torch.float32, torch.float16, torch.bfloat16):
             raise RuntimeError(f"gate_topk: k={k}, dtype={logits.dtype} is outside what the kernel takes "
                                "(k <= 8; float32, float16, bfloat16)")
+        if logits.dim() == 2:
+            return GateTopK.apply(logits, k, softmax)
         lead = logits.shape[:-1]
-        val, idx = GateTopK.apply(logits.reshape(-1, logits.shape[-1]), k)
+        val, idx = GateTopK.apply(logits.reshape(-1, logits.shape[-1]), k, softmax)
         return val.reshape(*lead, k), idx.reshape(*lead, k)
-    return torch.topk(logits, k=k, dim=-1, largest=True, sorted=True)       # CPU tensors: module set-up and tests only
+    val, idx = torch.topk(logits, k=k, dim=-1, largest=True, sorted=True)       # CPU tensors: module set-up and tests only
+    return (torch.softmax(val, dim=-1), idx) if softmax else (val, idx)
 
 
 class Slice(Function):

@@ -1,7 +1,6 @@
 """Linear gate with top-k selection (fmoe/gates/naive_gate.py:21-42)."""
 import torch
 import torch.nn as nn
-import torch.nn.functional as F
 
 from .base_gate import BaseGate
 from ..functions import gate_topk
@@ -24,10 +23,8 @@ class NaiveGate(BaseGate):
 
     def forward(self, inp, return_all_scores=False):
         gate = self.gate(inp)
-        top_val, top_idx = gate_topk(gate, self.top_k)
+        top_val, top_idx = gate_topk(gate, self.top_k, softmax=bool(self.softmax_scores))
         top_val = top_val.view(-1, self.top_k)
-        if self.softmax_scores:
-            top_val = F.softmax(top_val, dim=-1)
         if return_all_scores:
             return top_idx, top_val, gate
         return top_idx, top_val

@@ -88,6 +88,15 @@ int fmoe_gate_topk(const void* logits, int64_t n_tokens, int32_t n_expert_total,
 int fmoe_gate_topk_backward(const void* grad_values, const int64_t* indices, int64_t n_tokens,
                             int32_t n_expert_total, int32_t k, int32_t dtype, void* grad_logits,
                             fmoe_stream_t stream);
+/* The same selection with the softmax over the k selected logits (computed in
+ * fp32, rounded to dtype) as values, and its backward:
+ *   grad_logits[t, indices[t,j]] = probs[t,j] * (grad_probs[t,j] - sum_i probs[t,i] grad_probs[t,i]),
+ * zero elsewhere; probs are the values of the forward. */
+int fmoe_gate_topk_softmax(const void* logits, int64_t n_tokens, int32_t n_expert_total, int32_t k,
+                           int32_t dtype, void* probs, int64_t* indices, fmoe_stream_t stream);
+int fmoe_gate_topk_softmax_backward(const void* grad_probs, const void* probs, const int64_t* indices,
+                                    int64_t n_tokens, int32_t n_expert_total, int32_t k, int32_t dtype,
+                                    void* grad_logits, fmoe_stream_t stream);
 
 /* ------------------------------------------------------------------------
  * Routing: counting, bucketing, capacity            (integer work, bit-exact)

@@ -86,3 +86,26 @@ def test_hooks_are_called(act):
     m.expert_fn, plain = (lambda inp, *a: (out.append(inp.shape), plain(inp, *a))[1]), m.expert_fn
     m(x)
     assert out == [(40, 256)]
+
+
+@pytest.mark.parametrize("E,k", [(2, 2), (16, 1), (32, 8), (33, 4), (200, 3)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16, torch.bfloat16])
+def test_gate_softmax_in_the_selection(E, k, dtype):
+    """Scores and logit gradients of the fused softmax against torch on the library's own selection."""
+    from fastermoe_b200.functions import gate_topk
+    torch.manual_seed(E + k)
+    logits = (torch.randn(301, E, device="cuda") * 3).to(dtype)
+    logits[0], logits[1, 0], logits[2] = float("-inf"), float("nan"), 0
+    logits[3, 0], logits[4, 1] = float("inf"), float("-inf")
+    a, b = logits.clone().requires_grad_(True), logits.clone().requires_grad_(True)
+    val, idx = gate_topk(a, k, softmax=True)
+    raw, idx2 = gate_topk(b, k)
+    assert torch.equal(idx, idx2)
+    want = torch.softmax(raw, -1)
+    eps = torch.finfo(dtype).eps
+    torch.testing.assert_close(val, want, rtol=2 * eps, atol=1e-6, equal_nan=True)
+    g = torch.randn(301, k, device="cuda").to(dtype)
+    val.backward(g)
+    want.backward(g)
+    # products and a difference of the same rounded scores: a few roundings of the largest term
+    torch.testing.assert_close(a.grad, b.grad, rtol=4 * eps, atol=4 * eps, equal_nan=True)
