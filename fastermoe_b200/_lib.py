@@ -85,6 +85,7 @@ _SIGS = {
     "fmoe_count_and_pos_static": (I32, [P, I64, I32, P, P, P, P, P]),
     "fmoe_limit_by_capacity": (I32, [P, P, P, I32, I32, P]),
     "fmoe_prune_gate_by_capacity": (I32, [P, P, P, I64, I32, P, P]),
+    "fmoe_limit_and_prune": (I32, [P, P, P, P, I64, I32, P, P]),
     "fmoe_local_scatter": (I32, [P, P, P, I64, I64, I64, I32, P]),
     "fmoe_local_gather": (I32, [P, P, P, I64, I64, I64, P, P]),
     "fmoe_local_gather_inv": (I32, [P, P, P, I64, I64, P]),

@@ -233,6 +233,7 @@ finalize_kernel(int mode, int n_expert, int32_t* __restrict__ totals, int32_t* _
             const int32_t l = inout[e];
             limit[e] = l;
             inout[e] = l - totals[e];
+            if (lec64) lec64[e] = max(0, min(l, totals[e]));
             seg_start[e] = 0;
         }
         return;
@@ -422,6 +423,7 @@ bucket_cluster_kernel(int mode, const int64_t* __restrict__ gate, int64_t n, int
                 inout[e] = seg[e];
             } else {
                 inout[e] = lim[e] - total[e];
+                if (lec64) lec64[e] = max(0, min(lim[e], total[e]));     // entries kept
             }
         }
         if (mode == MODE_COUNT_POS && offsets && threadIdx.x == 0) offsets[n_expert] = s_grand;
@@ -639,6 +641,15 @@ extern "C" int fmoe_prune_gate_by_capacity(const int64_t* gate_idx, int64_t* new
     FMOE_REQUIRE(n == 0 || new_gate_idx != nullptr, "prune_gate_by_capacity: output pointer is null");
     return run_bucket(MODE_PRUNE, gate_idx, n, n_expert_total, scratch, nullptr, nullptr, ec, nullptr,
                       nullptr, new_gate_idx, (cudaStream_t)stream);
+}
+
+extern "C" int fmoe_limit_and_prune(const int64_t* gate_idx, int64_t* new_gate_idx, int32_t* capacity, int64_t* granted,
+                                    int64_t n, int32_t n_expert, void* scratch, fmoe_stream_t stream) {
+    if (int rc = check_routing_args(gate_idx, n, n_expert)) return rc;
+    FMOE_REQUIRE(capacity != nullptr && granted != nullptr, "limit_and_prune: capacity or granted pointer is null");
+    FMOE_REQUIRE(n == 0 || new_gate_idx != nullptr, "limit_and_prune: output pointer is null");
+    return run_bucket(MODE_PRUNE, gate_idx, n, n_expert, scratch, granted, nullptr, capacity, nullptr, nullptr, new_gate_idx,
+                      (cudaStream_t)stream);
 }
 
 extern "C" int fmoe_limit_by_capacity(const int64_t* ec, int32_t* cap, int64_t* eca, int32_t n_expert,

@@ -233,6 +233,20 @@ def prune_gate_by_capacity(gate_idx, expert_count, n_expert, n_worker):
     return out
 
 
+def limit_and_prune(gate_idx, capacity, n_expert):
+    """Capacity limiting on one worker: (granted int64 [E], new gate tensor); consumes ``capacity`` (int32 [E])."""
+    _check_cuda(gate_idx, capacity)
+    assert gate_idx.dtype == torch.int64 and capacity.dtype == torch.int32 and capacity.numel() == n_expert
+    out = torch.empty_like(gate_idx)
+    granted = torch.empty(n_expert, dtype=torch.int64, device=gate_idx.device)
+    n = gate_idx.numel()
+    with _device_of(gate_idx.device):
+        scratch = _routing_scratch(n, n_expert, gate_idx.device)
+        _run("limit_and_prune", lib.fmoe_limit_and_prune, _ptr(gate_idx), _ptr(out), _ptr(capacity), _ptr(granted), n, n_expert,
+             _ptr(scratch), _stream())
+    return granted, out
+
+
 # ---------------------------------------------------------------------------
 # parallel_linear: cuda/fmoe_cuda.cpp:57-69
 # ---------------------------------------------------------------------------

@@ -22,19 +22,17 @@ def limit_by_capacity(topk_idx, num_expert, world_size, capacity):
             cap = capacity.to(device=topk_idx.device, dtype=torch.int32).reshape(num_expert).clone()
         else:
             cap = torch.full((num_expert,), int(capacity), dtype=torch.int32, device=topk_idx.device)
+        if world_size == 1:
+            # every source is local: no grants to exchange, one pass does it all
+            granted, pruned = fmoe_native.limit_and_prune(topk_idx.contiguous(), cap, num_expert)
+            return granted, granted, pruned
         lec32 = torch.zeros(n_tot, dtype=torch.int32, device=topk_idx.device)
         fmoe_native.expert_count(topk_idx.reshape(-1).contiguous(), lec32)
         lec = lec32.long()
-        if world_size > 1:
-            _, _, gec = fmoe_native.expert_exchange(lec, num_expert, world_size)
-        else:
-            gec = lec
+        _, _, gec = fmoe_native.expert_exchange(lec, num_expert, world_size)
         new_gec = fmoe_native.limit_by_capacity(gec, cap, num_expert, world_size)
-        if world_size > 1:
-            # Sending the grants back is the same transpose as the count exchange.
-            _, _, new_lec = fmoe_native.expert_exchange(new_gec, num_expert, world_size)
-        else:
-            new_lec = new_gec
+        # Sending the grants back is the same transpose as the count exchange.
+        _, _, new_lec = fmoe_native.expert_exchange(new_gec, num_expert, world_size)
         pruned = fmoe_native.prune_gate_by_capacity(topk_idx.contiguous(), new_lec.to(torch.int32),
                                                     num_expert, world_size)
     return new_lec, new_gec, pruned

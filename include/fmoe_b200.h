@@ -179,6 +179,14 @@ int fmoe_prune_gate_by_capacity(const int64_t* gate_idx, int64_t* new_gate_idx,
                                 int32_t* ec, int64_t n, int32_t n_expert_total,
                                 void* scratch, fmoe_stream_t stream);
 
+/* Capacity limiting where every source is local (one worker): the counting,
+ * fmoe_limit_by_capacity and fmoe_prune_gate_by_capacity in one pass.
+ *   new_gate_idx[i] = gate_idx[i] while its expert has accepted fewer than
+ *       capacity[e] entries before it (lowest flat index first), else -1
+ *   granted[e] (int64) = entries kept; capacity[e] -= entries that asked. */
+int fmoe_limit_and_prune(const int64_t* gate_idx, int64_t* new_gate_idx, int32_t* capacity, int64_t* granted,
+                         int64_t n, int32_t n_expert, void* scratch, fmoe_stream_t stream);
+
 /* ------------------------------------------------------------------------
  * Token permutation                                  (byte copies, bit-exact)
  * ---------------------------------------------------------------------- */

@@ -109,3 +109,19 @@ def test_gate_softmax_in_the_selection(E, k, dtype):
     want.backward(g)
     # products and a difference of the same rounded scores: a few roundings of the largest term
     torch.testing.assert_close(a.grad, b.grad, rtol=4 * eps, atol=4 * eps, equal_nan=True)
+
+
+@pytest.mark.parametrize("n,E,cap", [(1, 1, 0), (5000, 16, 100), (5000, 16, 10 ** 6), (300000, 7, 20000)])
+def test_limit_and_prune(n, E, cap):
+    from fastermoe_b200 import fmoe_cuda as fc
+    g = np.random.default_rng(n).integers(-1, E, n)
+    left = torch.full((E,), cap, dtype=torch.int32, device="cuda")
+    granted, pruned = fc.limit_and_prune(torch.from_numpy(g).cuda(), left, E)
+    want, seen = g.copy(), np.zeros(E, dtype=np.int64)
+    for i, e in enumerate(g):
+        if e >= 0:
+            want[i] = e if seen[e] < cap else -1
+            seen[e] += 1
+    assert (pruned.cpu().numpy() == want).all()
+    assert (granted.cpu().numpy() == np.minimum(seen, cap)).all()
+    assert (left.cpu().numpy() == cap - seen).all()
