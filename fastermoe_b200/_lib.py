@@ -12,7 +12,7 @@ _HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(_HERE, "libfmoe_b200.so")
 
 F32, F16, BF16 = 0, 1, 2
-ACT_NONE, ACT_RELU, ACT_GELU = 0, 1, 2
+ACT_NONE, ACT_RELU, ACT_GELU, ACT_SILU = 0, 1, 2, 3
 GEMM_FORMS = {"auto": 0, "pair": 1, "tc1": 2, "simt": 3}
 MAX_EXPERTS = 4096
 

@@ -68,6 +68,7 @@ template <> __device__ __forceinline__ __nv_bfloat16 from_float<__nv_bfloat16>(f
 __device__ __forceinline__ float apply_act(float v, int act) {
     if (act == FMOE_ACT_RELU) return v > 0.f ? v : 0.f;
     if (act == FMOE_ACT_GELU) return 0.5f * v * (1.f + erff(v * 0.70710678118654752440f));
+    if (act == FMOE_ACT_SILU) return v / (1.f + expf(-v));
     return v;
 }
 // d act(v) / dv, for the exact (erf) GELU that torch.nn.GELU() computes and for
@@ -80,15 +81,22 @@ __device__ __forceinline__ float act_grad(float v, int act) {
         float pdf = 0.39894228040143267794f * __expf(-0.5f * v * v);
         return cdf + v * pdf;
     }
+    if (act == FMOE_ACT_SILU) {
+        const float s = 1.f / (1.f + expf(-v));
+        return s * (1.f + v * (1.f - s));
+    }
     return 1.f;
 }
 
+// Activations whose forward saves the derivative itself for the backward.
+__host__ __device__ constexpr bool saves_derivative(int act) { return act == FMOE_ACT_GELU || act == FMOE_ACT_SILU; }
+
 // Factor that the backward multiplies into the input gradient, from the buffer the
 // forward saved: for ReLU the buffer is the activation output (gradient is zero where
-// it is <= 0, cuda/fused_compute.cuh:36-44); for GELU it is the derivative itself.
+// it is <= 0, cuda/fused_compute.cuh:36-44); for GELU and SiLU it is the derivative itself.
 __device__ __forceinline__ float saved_act_grad(float saved, int act) {
     if (act == FMOE_ACT_RELU) return saved > 0.f ? 1.f : 0.f;
-    if (act == FMOE_ACT_GELU) return saved;
+    if (saves_derivative(act)) return saved;
     return 1.f;
 }
 

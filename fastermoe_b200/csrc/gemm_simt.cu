@@ -269,7 +269,7 @@ rows_gemm_kernel(const T* __restrict__ a, const T* __restrict__ w, const T* __re
 #pragma unroll
                     for (int j = 0; j < 4; ++j) q[j] += bv[j];
                 }
-                if (pre_out && act == FMOE_ACT_GELU) {
+                if (pre_out && saves_derivative(act)) {
                     float g[4];
 #pragma unroll
                     for (int j = 0; j < 4; ++j) g[j] = act_grad(q[j], act);

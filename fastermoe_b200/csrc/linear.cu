@@ -18,7 +18,7 @@ int check_common(int64_t n_rows, int64_t in_feat, int64_t out_feat, int n_expert
                  "linear: bad sizes rows=%lld in=%lld out=%lld experts=%d", (long long)n_rows,
                  (long long)in_feat, (long long)out_feat, n_expert);
     FMOE_REQUIRE(dtype_size(dtype) != 0, "linear: unknown dtype %d", dtype);
-    FMOE_REQUIRE(act >= FMOE_ACT_NONE && act <= FMOE_ACT_GELU, "linear: unknown activation %d", act);
+    FMOE_REQUIRE(act >= FMOE_ACT_NONE && act <= FMOE_ACT_SILU, "linear: unknown activation %d", act);
     FMOE_REQUIRE(seg != nullptr, "linear: seg_offsets pointer is null");
     return 0;
 }

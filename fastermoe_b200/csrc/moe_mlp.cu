@@ -57,7 +57,7 @@ struct Rows {
         Carver c{(char*)base};
         x = c.take(l.rows * l.row_d);
         h = c.take(l.rows * l.row_h);
-        pre = a.keep && a.activation > FMOE_ACT_RELU ? c.take(l.rows * l.row_h) : nullptr;
+        pre = a.keep && saves_derivative(a.activation) ? c.take(l.rows * l.row_h) : nullptr;
         y = a.keep ? c.take(l.rows * l.row_d) : x;
         bytes = c.at;
     }

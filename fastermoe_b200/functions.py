@@ -544,6 +544,7 @@ class PlannedExchange:
         return fmoe_cuda.peer_gather_planned(buf, self.plan, out_rows)
 
 
+_SAVES_DERIVATIVE = (_lib.ACT_GELU, _lib.ACT_SILU)       # their forward keeps the derivative for the backward
 _ACT_CODES = {"none": _lib.ACT_NONE, "relu": _lib.ACT_RELU, "gelu": _lib.ACT_GELU}
 
 
@@ -572,7 +573,7 @@ class FusedExpertMLP(Function):
         """``keep``: a backward may follow.  ``exch``: the PlannedExchange whose scatter produced ``x`` (and whose scatter of the output
         gradient will produce ``grad_y``); a pending arrival of it is waited for tile by tile."""
         x = x.contiguous()
-        want_pre = keep and act == _lib.ACT_GELU and (x.requires_grad or w1.requires_grad)
+        want_pre = keep and act in _SAVES_DERIVATIVE and (x.requires_grad or w1.requires_grad)
         arrival = exch.take_pending() if exch is not None else None
         h, pre = fmoe_cuda.linear_forward_act(x, offsets, w1, b1, act, want_pre=want_pre, arrival=arrival)
         y = x.new_empty((x.shape[0], w2.shape[1]))
@@ -592,7 +593,7 @@ class FusedExpertMLP(Function):
         act_pre = None
         if act == _lib.ACT_RELU:
             act_pre = h
-        elif act == _lib.ACT_GELU:
+        elif act in _SAVES_DERIVATIVE:
             act_pre = pre
         # The first layer's bias gradient is the column sum of gh: the input-gradient kernel of the
         # second layer returns it, so the first layer's backward does not read gh once more for it.

@@ -3,7 +3,9 @@ import os
 
 import torch
 import torch.nn as nn
+import torch.nn.functional as F
 
+from . import _lib
 from .gates import NaiveGate
 from .layers import FMoE, FMoELinear
 from .functions import FusedExpertMLP, ExpertCounts, activation_code
@@ -17,13 +19,19 @@ POLICY_CONSTANTS = {
 }
 
 
+def _plain(module, cls):
+    """True when calling ``module`` does what ``cls``'s forward does and nothing else."""
+    return (type(module) is cls and "forward" not in module.__dict__ and module._compiled_call_impl is None and
+            not (module._forward_hooks or module._forward_pre_hooks or module._backward_hooks or module._backward_pre_hooks))
+
+
 _KERNEL_DTYPES = (torch.float32, torch.float16, torch.bfloat16)
 
 
 class _Expert(nn.Module):
     r"""All experts of one worker as two grouped linear layers with an activation
-    in between (fmoe/transformer.py:10-30).  When the activation is ReLU or
-    exact GELU it is applied inside the GEMM epilogues."""
+    in between (fmoe/transformer.py:10-30).  When the activation is ReLU,
+    exact GELU or (on one GPU) SiLU it is applied inside the GEMM epilogues."""
 
     def __init__(self, num_expert, d_model, d_hidden, activation, rank=0, bias=True):
         super().__init__()
@@ -36,14 +44,22 @@ class _Expert(nn.Module):
         exchange that are still arriving (and later on the arriving output gradient)."""
         return inp.is_cuda and activation_code(self.activation) is not None
 
+    def _kernel_code(self):
+        """Code of the activation that the products' epilogues apply, or None.  SiLU is among them as long as the
+        three modules are called by nobody's hook: each is a call of its own otherwise."""
+        code = activation_code(self.activation)
+        if code is None and (self.activation is F.silu or _plain(self.activation, nn.SiLU)) and \
+                _plain(self.htoh4, FMoELinear) and _plain(self.h4toh, FMoELinear) and \
+                not torch.nn.modules.module._has_any_global_hook():
+            return _lib.ACT_SILU
+        return code
+
     def whole_layer_operands(self, inp):
         """(activation code, w1, b1, w2, b2) when nothing can tell a call of forward() from the fused layer call on
         the same parameters; else None."""
-        if (type(self) is not _Expert or "forward" in self.__dict__ or self._forward_hooks or self._forward_pre_hooks or
-                self._backward_hooks or self._backward_pre_hooks or self._compiled_call_impl is not None or
-                torch.nn.modules.module._has_any_global_hook()):
+        if not _plain(self, _Expert) or torch.nn.modules.module._has_any_global_hook():
             return None
-        code = activation_code(self.activation)
+        code = self._kernel_code()
         up, down = self.htoh4, self.h4toh
         w1, b1, w2, b2 = up.weight, up.bias, down.weight, down.bias
         if code is None or inp.dtype not in _KERNEL_DTYPES or inp.dim() != 2 or inp.shape[1] != w1.shape[2]:
@@ -54,8 +70,8 @@ class _Expert(nn.Module):
         return code, w1, b1, w2, b2
 
     def forward(self, inp, fwd_expert_count):
-        code = activation_code(self.activation)
         exch = getattr(fwd_expert_count, "exchange", None)
+        code = self._kernel_code() if exch is None else activation_code(self.activation)
         if code is None or not inp.is_cuda:
             if exch is not None:
                 exch.flush()

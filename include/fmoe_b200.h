@@ -41,7 +41,7 @@ enum {
 };
 
 enum { FMOE_F32 = 0, FMOE_F16 = 1, FMOE_BF16 = 2 };
-enum { FMOE_ACT_NONE = 0, FMOE_ACT_RELU = 1, FMOE_ACT_GELU = 2 };
+enum { FMOE_ACT_NONE = 0, FMOE_ACT_RELU = 1, FMOE_ACT_GELU = 2, FMOE_ACT_SILU = 3 };
 
 const char* fmoe_last_error_string(void);
 /* Library version, and the compute capability it was built for (100). */
@@ -286,7 +286,7 @@ int fmoe_linear_forward(const void* x, const void* weight, const void* bias,
  * derivative of the activation that produced x before it is stored (the
  * reference runs this as a separate kernel, cuda/fused_compute.cuh:155, or
  * leaves it to autograd).  For FMOE_ACT_RELU act_pre is the activation OUTPUT
- * (the factor is 1 where it is > 0); for FMOE_ACT_GELU it is the derivative
+ * (the factor is 1 where it is > 0); for FMOE_ACT_GELU and FMOE_ACT_SILU it is the derivative
  * buffer that fmoe_linear_forward wrote through pre_act.
  * accumulate != 0 adds into dW/db instead of overwriting them (what the smart
  * schedule's later pipeline steps do, cuda/fused_compute.cuh:120). */

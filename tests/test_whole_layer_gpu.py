@@ -5,7 +5,7 @@ import torch
 
 pytestmark = pytest.mark.gpu
 
-ACTS = {"gelu": torch.nn.GELU, "relu": torch.nn.ReLU}
+ACTS = {"gelu": torch.nn.GELU, "relu": torch.nn.ReLU, "silu": torch.nn.SiLU}
 
 
 def make(T, d, h, E, k, act="gelu", dtype=torch.bfloat16, bias=True, softmax=True, seed=0):
@@ -59,9 +59,9 @@ def test_partial_gradients():
     assert torch.equal(got[1], want[1]) and m.experts.htoh4.weight.grad is None
     assert torch.equal(m.gate.gate.weight.grad, want[2 + [n for n, _ in m.named_parameters()].index("gate.gate.weight")])
     m.experts.requires_grad_(True)
+    m.zero_grad()
     m(x.detach()).backward(g)
-    for (n, p), w in zip(m.named_parameters(), want[2:]):
-        torch.testing.assert_close(p.grad, w if n.startswith("gate") else p.grad)
+    assert all(torch.equal(p.grad, w) for p, w in zip(m.parameters(), want[2:]))
     m.zero_grad()
     m.requires_grad_(False)
     x.grad = None
@@ -69,7 +69,7 @@ def test_partial_gradients():
     assert torch.equal(x.grad, want[1])
 
 
-@pytest.mark.parametrize("act", ["gelu"])
+@pytest.mark.parametrize("act", ["gelu", "silu"])
 def test_hooks_are_called(act):
     m, x = make(20, 256, 512, 4, 2, act)
     base = m(x)
@@ -82,10 +82,40 @@ def test_hooks_are_called(act):
     torch.testing.assert_close(out, base, rtol=2e-2, atol=2e-2)
     for h in hooks:
         h.remove()
-    out = m.experts_out = []
-    m.expert_fn, plain = (lambda inp, *a: (out.append(inp.shape), plain(inp, *a))[1]), m.expert_fn
+    rows, plain = [], m.expert_fn
+    m.expert_fn = lambda inp, *a: (rows.append(tuple(inp.shape)), plain(inp, *a))[1]
     m(x)
-    assert out == [(40, 256)]
+    assert rows == [(40, 256)]
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("d,h", [(256, 320), (72, 200)])
+def test_silu_against_fp32(dtype, d, h):
+    """Layer with SiLU against plain autograd on the same (rounded) tensors in fp64; bounds as for the other
+    activations: fp32 1e-5 of a typical element, bf16 a few of its roundings."""
+    T, E, k = 90, 4, 2
+    m, x = make(T, d, h, E, k, "silu", dtype)
+    g = torch.randn(T, d, device="cuda").to(dtype)
+    out, gx, *grads = step(m, x, g)
+    with torch.no_grad():
+        idx, _ = m.gate(x)
+    leaves = {n: p.detach().double().requires_grad_(True) for n, p in m.named_parameters()}
+    xr = x.detach().double().requires_grad_(True)
+    logits = xr @ leaves["gate.gate.weight"].t() + leaves["gate.gate.bias"]
+    score = torch.softmax(torch.gather(logits, 1, idx), 1)
+    rows = []
+    for t in range(T):
+        acc = 0
+        for j in range(k):
+            e = int(idx[t, j])
+            mid = torch.nn.functional.silu(leaves["experts.htoh4.weight"][e] @ xr[t] + leaves["experts.htoh4.bias"][e])
+            acc = acc + score[t, j] * (leaves["experts.h4toh.weight"][e] @ mid + leaves["experts.h4toh.bias"][e])
+        rows.append(acc)
+    want = torch.stack(rows)
+    want.backward(g.double())
+    rel = 1e-5 if dtype == torch.float32 else 2e-2
+    for got, ref in [(out, want.detach()), (gx, xr.grad)] + [(a, leaves[n].grad) for a, (n, _) in zip(grads, m.named_parameters())]:
+        assert float((got.double() - ref).norm()) <= rel * float(ref.norm())
 
 
 @pytest.mark.parametrize("E,k", [(2, 2), (16, 1), (32, 8), (33, 4), (200, 3)])
