@@ -30,6 +30,7 @@
 #include "gemm.h"
 #include <cuda.h>
 #include <algorithm>
+#include <cooperative_groups.h>
 #include <atomic>
 #include <cstdlib>
 #include <mutex>
@@ -1633,26 +1634,34 @@ bool shape_ok(int64_t n_rows, int64_t in_feat, int64_t out_feat, int n_expert, i
            (int64_t)n_expert * out_feat < ((int64_t)1 << 31);
 }
 
-// Column sums of dY per expert segment (bias gradient), fp32 accumulate.
-// Block = CL column lanes (8 columns each, one 16-byte load) x 256/CL row lanes;
-// every thread keeps four independent row loads in flight.  CL = 16 (128 columns per
-// block) for wide outputs, 8 (64 columns) when that gives too few blocks.
-template <bool BF16, int CL>
+// Column sums of dY per expert segment (bias gradient), fp32 accumulate.  A cluster of kBiasSplit blocks per
+// (128 columns, expert): each block sums a share of the segment's rows (16 column lanes of one 16-byte load each x 16
+// row lanes, four rows in flight per thread), the first one adds the shares, read through distributed shared memory, in
+// order.  One block per expert was bound by the longest segment: 16384 rows of 32 skewed experts, 2048 columns, took
+// 256 us, 50 now.
+constexpr int kBiasSplit = 8;
+
+template <bool BF16>
 __global__ void __launch_bounds__(256)
 bias_grad_tc_kernel(const uint16_t* __restrict__ dy, const int64_t* __restrict__ seg,
                     const __grid_constant__ HostSegs hs, uint16_t* __restrict__ db, int64_t n_rows, int out_feat, int accumulate) {
-    constexpr int RL = 256 / CL, COLS = CL * 8;
+    namespace cg = cooperative_groups;
+    cg::cluster_group cluster = cg::this_cluster();
+    constexpr int CL = 16, RL = 256 / CL, COLS = CL * 8;
     __shared__ float red[RL][COLS + 1];
+    __shared__ float share[COLS];
     const int e = blockIdx.y;
     const int cl = threadIdx.x % CL, ry = threadIdx.x / CL;
     const int col = blockIdx.x * COLS + cl * 8;
     int64_t lo, hi;
     safe_seg_range(seg, hs, e, n_rows, lo, hi);
+    const int64_t per = (hi - lo + kBiasSplit - 1) / kBiasSplit;
+    const int64_t my_lo = lo + blockIdx.z * per, my_hi = min(hi, my_lo + per);
     float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
     if (col < out_feat) {
         const uint16_t* base = dy + col;
-        int64_t m = lo + ry;
-        for (; m + 3 * RL < hi; m += 4 * RL) {
+        int64_t m = my_lo + ry;
+        for (; m + 3 * RL < my_hi; m += 4 * RL) {
             uint4 v[4];
 #pragma unroll
             for (int u = 0; u < 4; ++u) v[u] = __ldg(reinterpret_cast<const uint4*>(base + (m + RL * u) * out_feat));
@@ -1666,7 +1675,7 @@ bias_grad_tc_kernel(const uint16_t* __restrict__ dy, const int64_t* __restrict__
                 }
             }
         }
-        for (; m < hi; m += RL) {
+        for (; m < my_hi; m += RL) {
             const uint4 v = __ldg(reinterpret_cast<const uint4*>(base + m * out_feat));
             const uint32_t w[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
@@ -1680,17 +1689,25 @@ bias_grad_tc_kernel(const uint16_t* __restrict__ dy, const int64_t* __restrict__
     for (int i = 0; i < 8; ++i) red[ry][cl * 8 + i] = acc[i];
     __syncthreads();
     if (threadIdx.x < COLS) {
+        float t = 0.f;
+#pragma unroll
+        for (int i = 0; i < RL; ++i) t += red[i][threadIdx.x];
+        share[threadIdx.x] = t;
+    }
+    cluster.sync();
+    if (blockIdx.z == 0 && threadIdx.x < COLS) {
         const int c = blockIdx.x * COLS + threadIdx.x;
         if (c < out_feat) {
             float t = 0.f;
 #pragma unroll
-            for (int i = 0; i < RL; ++i) t += red[i][threadIdx.x];
+            for (int r = 0; r < kBiasSplit; ++r) t += *cluster.map_shared_rank(share + threadIdx.x, r);
             uint16_t* o = db + (size_t)e * out_feat + c;
             if (accumulate) t += cvt_in<BF16>(*o);
             const uint32_t packed = cvt_pack<BF16>(t, 0.f);
             *o = (uint16_t)(packed & 0xffff);
         }
     }
+    cluster.sync();      // no block leaves while its share may still be read
 }
 
 // Adds up the per-block partial column sums that the input-gradient kernel left in the
@@ -1704,30 +1721,48 @@ colsum_finish_kernel(const float* __restrict__ partial, const int64_t* __restric
     __shared__ float2 part[4][128];
     const int e = blockIdx.y, q = threadIdx.y;
     const int col = (blockIdx.x * 128 + threadIdx.x) * 2;
-    // the same (clamped) ranges and 32-row block numbering as the kernel that wrote the partial sums
-    int base = 0;
-    int64_t lo = 0, hi = 0, prev_hi = 0;
-    for (int j = 0; j <= e; ++j) {
-        if (j) base += (int)((hi - lo + 31) >> 5);
-        lo = hs.n ? (int64_t)hs.lo[j] : seg[j];
-        hi = hs.n ? (int64_t)hs.hi[j] : seg[j + 1];
-        lo = min(max(lo, prev_hi), n_rows);
-        hi = min(max(hi, lo), n_rows);
-        prev_hi = hi;
+    // the same (clamped) ranges and 32-row block numbering as the kernel that wrote the partial sums, found by each warp
+    // with one round of loads per 32 experts
+    int base = 0, nb = 0, before = 0;
+    const int lane = threadIdx.x & 31;
+    for (int j0 = 0; j0 <= e; j0 += 32) {
+        const int j = j0 + lane;
+        int64_t raw_lo = 0, raw_hi = 0;
+        if (j <= e) {
+            raw_lo = hs.n ? (int64_t)hs.lo[j] : __ldg(seg + j);
+            raw_hi = hs.n ? (int64_t)hs.hi[j] : __ldg(seg + j + 1);
+        }
+        const int c_lo = (int)min(max(raw_lo, (int64_t)0), n_rows), c_hi = (int)min(max(raw_hi, (int64_t)0), n_rows);
+        int far = max(c_lo, c_hi);
+#pragma unroll
+        for (int off = 1; off < 32; off <<= 1) {
+            const int o = __shfl_up_sync(0xffffffffu, far, off);
+            if (lane >= off) far = max(far, o);
+        }
+        const int prev = __shfl_up_sync(0xffffffffu, far, 1);
+        const int lo = max(max(before, lane ? prev : 0), c_lo), hi = max(lo, c_hi);
+        before = max(before, __shfl_sync(0xffffffffu, far, 31));
+        int blocks = j <= e ? (hi - lo + 31) >> 5 : 0;
+        if (j0 + 32 > e) {                 // the round that holds e itself
+            nb = __shfl_sync(0xffffffffu, blocks, e - j0);
+            if (j == e) blocks = 0;
+        }
+#pragma unroll
+        for (int off = 16; off > 0; off >>= 1) blocks += __shfl_xor_sync(0xffffffffu, blocks, off);
+        base += blocks;
     }
-    const int nb = (int)((hi - lo + 31) >> 5);
     const int per = (nb + 3) >> 2;
     const int b0 = min(nb, q * per), b1 = min(nb, b0 + per);
     float t0 = 0.f, t1 = 0.f;
     if (col < n_cols) {
         const float* src = partial + (size_t)base * n_cols + col;
         int b = b0;
-        for (; b + 3 < b1; b += 4) {
-            const float2 v0 = *reinterpret_cast<const float2*>(src + (size_t)b * n_cols);
-            const float2 v1 = *reinterpret_cast<const float2*>(src + (size_t)(b + 1) * n_cols);
-            const float2 v2 = *reinterpret_cast<const float2*>(src + (size_t)(b + 2) * n_cols);
-            const float2 v3 = *reinterpret_cast<const float2*>(src + (size_t)(b + 3) * n_cols);
-            t0 += v0.x; t1 += v0.y; t0 += v1.x; t1 += v1.y; t0 += v2.x; t1 += v2.y; t0 += v3.x; t1 += v3.y;
+        for (; b + 7 < b1; b += 8) {
+            float2 v[8];
+#pragma unroll
+            for (int u = 0; u < 8; ++u) v[u] = *reinterpret_cast<const float2*>(src + (size_t)(b + u) * n_cols);
+#pragma unroll
+            for (int u = 0; u < 8; ++u) { t0 += v[u].x; t1 += v[u].y; }
         }
         for (; b < b1; ++b) {
             const float2 v = *reinterpret_cast<const float2*>(src + (size_t)b * n_cols);
@@ -1750,17 +1785,17 @@ colsum_finish_kernel(const float* __restrict__ partial, const int64_t* __restric
 
 template <bool BF16>
 int launch_bias_grad(const LinearBwdArgs& a, const HostSegs& hs, cudaStream_t st) {
-    const bool narrow = ceil_div(a.out_feat, 128) * a.n_expert < 2 * sm_count();
-    if (narrow) {
-        dim3 grid((unsigned)ceil_div(a.out_feat, 64), (unsigned)a.n_expert);
-        bias_grad_tc_kernel<BF16, 8><<<grid, 256, 0, st>>>((const uint16_t*)a.grad_y, a.seg_offsets, hs, (uint16_t*)a.grad_b,
-                                                            a.n_rows, (int)a.out_feat, a.accumulate);
-    } else {
-        dim3 grid((unsigned)ceil_div(a.out_feat, 128), (unsigned)a.n_expert);
-        bias_grad_tc_kernel<BF16, 16><<<grid, 256, 0, st>>>((const uint16_t*)a.grad_y, a.seg_offsets, hs, (uint16_t*)a.grad_b,
-                                                             a.n_rows, (int)a.out_feat, a.accumulate);
-    }
-    FMOE_CHECK_LAUNCH();
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)ceil_div(a.out_feat, 128), (unsigned)a.n_expert, kBiasSplit);
+    cfg.blockDim = dim3(256);
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 1; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = kBiasSplit;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    FMOE_CUDA_TRY(cudaLaunchKernelEx(&cfg, bias_grad_tc_kernel<BF16>, (const uint16_t*)a.grad_y, a.seg_offsets, hs,
+                                     (uint16_t*)a.grad_b, a.n_rows, (int)a.out_feat, a.accumulate));
     return 0;
 }
 
@@ -1824,57 +1859,24 @@ int tc_linear_forward(const LinearArgs& a, cudaStream_t st) {
                 : launch<MODE_FWD, false>(ma, mb, a.host_segs, p, max_tiles, a.n_rows, st, reserve, a.remote, a.push);
 }
 
-// A side stream and a pair of events per device, created on first use: the bias
-// gradient (an HBM-bound column sum with a small footprint) runs there, next to the
-// tensor-core kernels of the same call, instead of after them.
-struct SideStream {
-    cudaStream_t stream = nullptr;
-    cudaEvent_t fork = nullptr, join = nullptr;
-};
-int side_stream(SideStream** out) {
-    static SideStream pool[64];
-    static std::mutex mtx;
-    int dev = 0;
-    FMOE_CUDA_TRY(cudaGetDevice(&dev));
-    if (dev < 0 || dev >= 64) dev = 0;
-    std::lock_guard<std::mutex> lk(mtx);
-    SideStream& s = pool[dev];
-    if (!s.stream) {
-        FMOE_CUDA_TRY(cudaStreamCreateWithFlags(&s.stream, cudaStreamNonBlocking));
-        FMOE_CUDA_TRY(cudaEventCreateWithFlags(&s.fork, cudaEventDisableTiming));
-        FMOE_CUDA_TRY(cudaEventCreateWithFlags(&s.join, cudaEventDisableTiming));
-    }
-    *out = &s;
-    return 0;
-}
-
 int tc_linear_backward(const LinearBwdArgs& a, cudaStream_t st) {
     const bool bf16 = a.dtype == FMOE_BF16;
-    SideStream* side = nullptr;
-    const bool overlap_bias = a.grad_b && (a.grad_x || a.grad_w) && a.n_rows > 0;
-    // grad_y still arriving: only the input-gradient product may start; everything else (the bias
-    // gradient on the side stream included) is queued after the exchange has been closed
+    const HostSegs& hs = a.host_segs ? *a.host_segs : kNoSegs;
+    // grad_y still arriving: only the input-gradient product may start; everything else is queued after the
+    // exchange has been closed
     const bool arriving = a.arrival != nullptr;
     bool closed = !arriving;
     if (arriving && !(a.grad_x && a.n_rows > 0)) {
         if (a.after_input_grad) { if (int rc = a.after_input_grad(a.after_ctx)) return rc; }
         closed = true;
     }
-    auto queue_bias = [&]() -> int {
-        if (int rc = side_stream(&side)) return rc;
-        const HostSegs& hs = a.host_segs ? *a.host_segs : kNoSegs;
-        FMOE_CUDA_TRY(cudaEventRecord(side->fork, st));
-        FMOE_CUDA_TRY(cudaStreamWaitEvent(side->stream, side->fork, 0));
-        if (int rc = bf16 ? launch_bias_grad<true>(a, hs, side->stream) : launch_bias_grad<false>(a, hs, side->stream))
-            return rc;
-        FMOE_CUDA_TRY(cudaEventRecord(side->join, side->stream));
-        return 0;
+    // The bias gradient comes first, while L2 still holds part of the rows the caller has just written.  (On a stream
+    // of its own beside the products, it got its SMs only when the persistent input-gradient product gave them up, and
+    // then kept the weight gradient from them.)
+    auto bias_grad = [&]() -> int {
+        return !a.grad_b ? 0 : bf16 ? launch_bias_grad<true>(a, hs, st) : launch_bias_grad<false>(a, hs, st);
     };
-    if (overlap_bias && !closed) {
-        // queued below, after the input-gradient product
-    } else if (overlap_bias) {
-        if (int rc = queue_bias()) return rc;
-    }
+    if (closed) { if (int rc = bias_grad()) return rc; }
     if (a.grad_x && a.n_rows > 0) {
         CUtensorMap ma, mb;
         const Form form = pick_form(MODE_DGRAD, a.n_rows, a.n_expert, a.in_feat, a.out_feat);
@@ -1919,10 +1921,9 @@ int tc_linear_backward(const LinearBwdArgs& a, cudaStream_t st) {
         if (!closed) {
             if (a.after_input_grad) { if (int rc = a.after_input_grad(a.after_ctx)) return rc; }
             closed = true;
-            if (overlap_bias) { if (int rc = queue_bias()) return rc; }
+            if (int rc = bias_grad()) return rc;
         }
         if (a.grad_x_colsum) {
-            const HostSegs& hs = a.host_segs ? *a.host_segs : kNoSegs;
             dim3 grid((unsigned)ceil_div(a.in_feat, 256), (unsigned)a.n_expert);
             if (bf16) colsum_finish_kernel<true><<<grid, dim3(128, 4), 0, st>>>((const float*)a.scratch, a.seg_offsets, hs,
                                                                                 (uint16_t*)a.grad_x_colsum, a.n_rows, (int)a.in_feat, 0);
@@ -1949,12 +1950,6 @@ int tc_linear_backward(const LinearBwdArgs& a, cudaStream_t st) {
         if (int rc = pair ? launch<MODE_WGRAD, true>(ma, mb, a.host_segs, p, max_tiles, (int64_t)a.n_expert * a.out_feat, st, reserve)
                           : launch<MODE_WGRAD, false>(ma, mb, a.host_segs, p, max_tiles, (int64_t)a.n_expert * a.out_feat, st, reserve))
             return rc;
-    }
-    if (overlap_bias) {
-        FMOE_CUDA_TRY(cudaStreamWaitEvent(st, side->join, 0));
-    } else if (a.grad_b) {
-        const HostSegs& hs = a.host_segs ? *a.host_segs : kNoSegs;
-        if (int rc = bf16 ? launch_bias_grad<true>(a, hs, st) : launch_bias_grad<false>(a, hs, st)) return rc;
     }
     return 0;
 }
