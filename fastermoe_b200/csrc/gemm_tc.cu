@@ -422,18 +422,6 @@ __device__ __forceinline__ void act_pairs(int act, float* v, float* g) {
         }
     }
 }
-__device__ __forceinline__ float gelu_fast(float x) {
-    f32x2 v, g;
-    gelu_pair<false>(pk(x, x), v, g);
-    float lo, hi;
-    unpk(v, lo, hi);
-    return lo;
-}
-__device__ __forceinline__ float act_fast(float v, int act) {
-    if (act == FMOE_ACT_RELU) return v > 0.f ? v : 0.f;
-    if (act == FMOE_ACT_GELU) return gelu_fast(v);
-    return v;
-}
 // Two 16-bit values of one 32-bit word as a packed fp32 pair.
 template <bool BF16> __device__ __forceinline__ f32x2 cvt_in2(uint32_t w) {
     if (BF16) return pk(__uint_as_float(w << 16), __uint_as_float(w & 0xffff0000u));
@@ -1125,9 +1113,9 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                             }
                         } else if (saves_derivative(p.act)) {
                             act_pairs<false, CW / 2>(p.act, v, nullptr);
-                        } else if (p.act != FMOE_ACT_NONE) {
+                        } else if (p.act == FMOE_ACT_RELU) {
 #pragma unroll
-                            for (int i = 0; i < CW; ++i) v[i] = act_fast(v[i], p.act);
+                            for (int i = 0; i < CW; ++i) v[i] = v[i] > 0.f ? v[i] : 0.f;
                         }
                     } else if (aux_src) {
 #pragma unroll
@@ -1273,9 +1261,9 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
                             }
                         } else if (saves_derivative(p.act)) {
                             act_pairs<false, CW / 2>(p.act, v, nullptr);
-                        } else if (p.act != FMOE_ACT_NONE) {
+                        } else if (p.act == FMOE_ACT_RELU) {
 #pragma unroll
-                            for (int i = 0; i < CW; ++i) v[i] = act_fast(v[i], p.act);
+                            for (int i = 0; i < CW; ++i) v[i] = v[i] > 0.f ? v[i] : 0.f;
                         }
                     } else if (MODE == MODE_DGRAD) {
                         if (p.act_pre && saves_derivative(p.act)) {
