@@ -113,6 +113,9 @@ _SIGS = {
     "fmoe_gate_topk_backward": (I32, [P, P, I64, I32, I32, I32, P, P]),
     "fmoe_gate_topk_softmax": (I32, [P, I64, I32, I32, I32, P, P, P]),
     "fmoe_gate_topk_softmax_backward": (I32, [P, P, P, I64, I32, I32, I32, P, P]),
+    "fmoe_balance_loss_scratch_bytes": (c_size_t, [I64, I32]),
+    "fmoe_balance_loss": (I32, [P, P, I64, I64, I32, I32, ctypes.c_float, P, P, P, P]),
+    "fmoe_balance_loss_backward": (I32, [P, P, P, I64, I32, I32, ctypes.c_float, P, P]),
     "fmoe_peer_plan": (I32, [P, P, I32, I32, I32, I32, P, POINTER(c_int32), P, POINTER(c_int32), I32, POINTER(c_int64)]),
     "fmoe_peer_enable": (I32, [P, I64, I64, P]),
     "fmoe_peer_pool_bytes": (I64, [P]),

@@ -217,3 +217,174 @@ extern "C" int fmoe_gate_topk_softmax_backward(const void* grad_probs, const voi
                                                void* grad_logits, fmoe_stream_t stream) {
     return topk_backward<true>(grad_probs, probs, indices, n_tokens, n_expert_total, k, dtype, grad_logits, (cudaStream_t)stream);
 }
+
+// ---- balance loss of the capacity gates ------------------------------------------------------------------------
+// Seventeen small torch operators (nine forward, eight backward) on [T, E] values were bound by their launches; two
+// kernels forward and one backward here (step of 8192 tokens with a capacity gate, 1024 x 4096, 16 experts: 1054 us
+// with the operators, 1014 with the kernels).  One warp per token: lane l holds the experts l, l + 32, ...
+namespace fmoe {
+namespace {
+
+constexpr int kBalMax = 256, kBalRegs = kBalMax / 32, kBalWarps = 8;
+int balance_blocks(int64_t n_tokens) { return (int)std::min<int64_t>(ceil_div(n_tokens, kBalWarps), 128); }
+
+// softmax of one row; the lanes' shares of it (zero past n_expert)
+template <typename T>
+__device__ __forceinline__ void warp_softmax(const T* __restrict__ row, int n_expert, int lane, float (&p)[kBalRegs]) {
+    float top = -INFINITY;
+#pragma unroll
+    for (int i = 0; i < kBalRegs; ++i) {
+        const int e = i * 32 + lane;
+        p[i] = e < n_expert ? to_float<T>(row[e]) : -INFINITY;
+        top = fmaxf(top, p[i]);
+    }
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, off));
+    float sum = 0.f;
+#pragma unroll
+    for (int i = 0; i < kBalRegs; ++i) {
+        p[i] = i * 32 + lane < n_expert ? expf(p[i] - top) : 0.f;     // (a row with NaN, or of -inf alone, becomes NaN)
+        sum += p[i];
+    }
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, off);
+    const float r = 1.f / sum;
+#pragma unroll
+    for (int i = 0; i < kBalRegs; ++i)
+        if (i * 32 + lane < n_expert) p[i] *= r;
+}
+
+// partial[block][e]: sum of the probabilities of the block's tokens; counts[block][e]: first choices
+template <typename T>
+__global__ void __launch_bounds__(kBalWarps * 32)
+balance_sums_kernel(const T* __restrict__ logits, const int64_t* __restrict__ first, int64_t stride, int64_t n_tokens,
+                    int n_expert, float* __restrict__ partial, int* __restrict__ counts) {
+    __shared__ float sums[kBalWarps][kBalMax];
+    __shared__ int hist[kBalMax];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    for (int e = threadIdx.x; e < n_expert; e += blockDim.x) hist[e] = 0;
+    __syncthreads();
+    float acc[kBalRegs] = {};
+    for (int64_t t = (int64_t)blockIdx.x * kBalWarps + warp; t < n_tokens; t += (int64_t)gridDim.x * kBalWarps) {
+        float p[kBalRegs];
+        warp_softmax<T>(logits + t * n_expert, n_expert, lane, p);
+#pragma unroll
+        for (int i = 0; i < kBalRegs; ++i) acc[i] += p[i];
+        if (lane == 0) {
+            const int64_t e = first[t * stride];
+            if (e >= 0 && e < n_expert) atomicAdd(hist + (int)e, 1);
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < kBalRegs; ++i) sums[warp][i * 32 + lane] = acc[i];
+    __syncthreads();
+    for (int e = threadIdx.x; e < n_expert; e += blockDim.x) {
+        float s = 0.f;
+#pragma unroll
+        for (int w = 0; w < kBalWarps; ++w) s += sums[w][e];
+        partial[(size_t)blockIdx.x * n_expert + e] = s;
+        counts[(size_t)blockIdx.x * n_expert + e] = hist[e];
+    }
+}
+
+__global__ void __launch_bounds__(kBalMax)
+balance_finish_kernel(const float* __restrict__ partial, const int* __restrict__ counts, int blocks, int64_t n_tokens,
+                      int n_expert, float scale, float* __restrict__ loss, float* __restrict__ share) {
+    __shared__ float terms[kBalMax];
+    const int e = threadIdx.x;
+    float term = 0.f;
+    if (e < n_expert) {
+        float s = 0.f;
+        int c = 0;
+#pragma unroll 8
+        for (int b = 0; b < blocks; ++b) {
+            s += partial[(size_t)b * n_expert + e];
+            c += counts[(size_t)b * n_expert + e];
+        }
+        const float part = (float)c / (float)n_tokens;
+        share[e] = part;
+        term = part * (s / (float)n_tokens);
+    }
+    terms[e] = term;
+    __syncthreads();
+    if (e == 0) {
+        float t = 0.f;
+        for (int i = 0; i < n_expert; ++i) t += terms[i];
+        *loss = t * scale;
+    }
+}
+
+template <typename T>
+__global__ void __launch_bounds__(kBalWarps * 32)
+balance_backward_kernel(const T* __restrict__ logits, const float* __restrict__ share, const float* __restrict__ grad_loss,
+                        int64_t n_tokens, int n_expert, float scale, T* __restrict__ grad) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int64_t t = (int64_t)blockIdx.x * kBalWarps + warp;
+    if (t >= n_tokens) return;
+    const float g = *grad_loss * scale / (float)n_tokens;
+    float p[kBalRegs], w[kBalRegs], dot = 0.f;
+    warp_softmax<T>(logits + t * n_expert, n_expert, lane, p);
+#pragma unroll
+    for (int i = 0; i < kBalRegs; ++i) {
+        const int e = i * 32 + lane;
+        w[i] = e < n_expert ? g * share[e] : 0.f;
+        dot = fmaf(p[i], w[i], dot);
+    }
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) dot += __shfl_xor_sync(0xffffffffu, dot, off);
+#pragma unroll
+    for (int i = 0; i < kBalRegs; ++i) {
+        const int e = i * 32 + lane;
+        if (e < n_expert) grad[t * n_expert + e] = from_float<T>(p[i] * (w[i] - dot));
+    }
+}
+
+int check_balance(const void* logits, int64_t n_tokens, int32_t n_expert, int32_t dtype) {
+    FMOE_REQUIRE(n_tokens > 0 && n_expert > 0 && n_expert <= kBalMax, "balance_loss: n_tokens=%lld n_expert=%d (1..%d)",
+                 (long long)n_tokens, n_expert, kBalMax);
+    FMOE_REQUIRE(dtype_size(dtype) > 0, "balance_loss: unknown dtype %d", dtype);
+    FMOE_REQUIRE(logits, "balance_loss: null pointer");
+    return 0;
+}
+
+}  // namespace
+}  // namespace fmoe
+
+extern "C" size_t fmoe_balance_loss_scratch_bytes(int64_t n_tokens, int32_t n_expert) {
+    return n_tokens > 0 && n_expert > 0 ? (size_t)balance_blocks(n_tokens) * (size_t)n_expert * 8 : 0;
+}
+
+extern "C" int fmoe_balance_loss(const void* logits, const int64_t* first_choice, int64_t choice_stride, int64_t n_tokens,
+                                 int32_t n_expert, int32_t dtype, float scale, float* loss, float* share, void* scratch,
+                                 fmoe_stream_t stream) {
+    if (int rc = check_balance(logits, n_tokens, n_expert, dtype)) return rc;
+    FMOE_REQUIRE(first_choice && loss && share && scratch, "balance_loss: null pointer");
+    cudaStream_t st = (cudaStream_t)stream;
+    const int blocks = balance_blocks(n_tokens);
+    float* partial = (float*)scratch;
+    int* counts = (int*)scratch + (size_t)blocks * n_expert;
+    switch (dtype) {
+        case FMOE_F32: balance_sums_kernel<float><<<blocks, kBalWarps * 32, 0, st>>>((const float*)logits, first_choice, choice_stride, n_tokens, n_expert, partial, counts); break;
+        case FMOE_F16: balance_sums_kernel<__half><<<blocks, kBalWarps * 32, 0, st>>>((const __half*)logits, first_choice, choice_stride, n_tokens, n_expert, partial, counts); break;
+        default: balance_sums_kernel<__nv_bfloat16><<<blocks, kBalWarps * 32, 0, st>>>((const __nv_bfloat16*)logits, first_choice, choice_stride, n_tokens, n_expert, partial, counts); break;
+    }
+    FMOE_CHECK_LAUNCH();
+    balance_finish_kernel<<<1, kBalMax, 0, st>>>(partial, counts, blocks, n_tokens, n_expert, scale, loss, share);
+    FMOE_CHECK_LAUNCH();
+    return 0;
+}
+
+extern "C" int fmoe_balance_loss_backward(const void* logits, const float* share, const float* grad_loss, int64_t n_tokens,
+                                          int32_t n_expert, int32_t dtype, float scale, void* grad_logits, fmoe_stream_t stream) {
+    if (int rc = check_balance(logits, n_tokens, n_expert, dtype)) return rc;
+    FMOE_REQUIRE(share && grad_loss && grad_logits, "balance_loss_backward: null pointer");
+    cudaStream_t st = (cudaStream_t)stream;
+    const unsigned blocks = (unsigned)ceil_div(n_tokens, kBalWarps);
+    switch (dtype) {
+        case FMOE_F32: balance_backward_kernel<float><<<blocks, kBalWarps * 32, 0, st>>>((const float*)logits, share, grad_loss, n_tokens, n_expert, scale, (float*)grad_logits); break;
+        case FMOE_F16: balance_backward_kernel<__half><<<blocks, kBalWarps * 32, 0, st>>>((const __half*)logits, share, grad_loss, n_tokens, n_expert, scale, (__half*)grad_logits); break;
+        default: balance_backward_kernel<__nv_bfloat16><<<blocks, kBalWarps * 32, 0, st>>>((const __nv_bfloat16*)logits, share, grad_loss, n_tokens, n_expert, scale, (__nv_bfloat16*)grad_logits); break;
+    }
+    FMOE_CHECK_LAUNCH();
+    return 0;
+}

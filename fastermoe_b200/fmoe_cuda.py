@@ -847,6 +847,34 @@ def gate_topk_backward(grad_values, indices, n_expert_total, probs=None):
     return out
 
 
+BALANCE_MAX_EXPERTS = 256
+
+
+def balance_loss(logits, first_choice, scale):
+    """(loss fp32 scalar, share fp32 [E]): scale * sum_e share_e * mean_t softmax(logits)_te, share_e the part of
+    the tokens whose ``first_choice`` (int64 [T], any stride) is e."""
+    _check_cuda(logits)
+    assert first_choice.is_cuda and first_choice.dtype == torch.int64 and first_choice.shape == logits.shape[:1]
+    n_tok, n_exp = logits.shape
+    loss = torch.empty((), dtype=torch.float32, device=logits.device)
+    share = torch.empty(n_exp, dtype=torch.float32, device=logits.device)
+    with _device_of(logits.device):
+        scratch = _scratch(lib.fmoe_balance_loss_scratch_bytes(n_tok, n_exp), logits.device)
+        _run("balance_loss", lib.fmoe_balance_loss, _ptr(logits), _ptr(first_choice), first_choice.stride(0), n_tok, n_exp,
+             _dtype_code(logits), float(scale), _ptr(loss), _ptr(share), _ptr(scratch), _stream())
+    return loss, share
+
+
+def balance_loss_backward(logits, share, grad_loss, scale):
+    """Gradient of balance_loss with respect to the logits."""
+    _check_cuda(logits, share, grad_loss)
+    out = torch.empty_like(logits)
+    with _device_of(logits.device):
+        _run("balance_loss_backward", lib.fmoe_balance_loss_backward, _ptr(logits), _ptr(share), _ptr(grad_loss),
+             logits.shape[0], logits.shape[1], _dtype_code(logits), float(scale), _ptr(out), _stream())
+    return out
+
+
 def count_and_pos(gate, n_expert_total, want_inv=True):
     """One-call form of count_by_gate's bucketing (fmoe/functions.py:19-41).
 

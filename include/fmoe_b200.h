@@ -98,6 +98,20 @@ int fmoe_gate_topk_softmax_backward(const void* grad_probs, const void* probs, c
                                     int64_t n_tokens, int32_t n_expert_total, int32_t k, int32_t dtype,
                                     void* grad_logits, fmoe_stream_t stream);
 
+/* Balance loss of the capacity gates (fmoe/gates/gshard_gate.py:27-35):
+ *   loss = scale * sum_e c_e m_e,  c_e = (tokens whose first choice is e) / n_tokens,
+ *   m_e = mean over tokens of softmax(logits[t,:])_e
+ * in fp32.  first_choice[t * choice_stride] is token t's first expert; entries
+ * outside [0, n_expert) count nowhere.  share [n_expert] receives c_e; scratch
+ * holds fmoe_balance_loss_scratch_bytes.  n_expert <= 256.
+ * Backward: grad_logits [n_tokens, n_expert] (dtype) from the scalar grad_loss (fp32, device). */
+size_t fmoe_balance_loss_scratch_bytes(int64_t n_tokens, int32_t n_expert);
+int fmoe_balance_loss(const void* logits, const int64_t* first_choice, int64_t choice_stride, int64_t n_tokens,
+                      int32_t n_expert, int32_t dtype, float scale, float* loss, float* share, void* scratch,
+                      fmoe_stream_t stream);
+int fmoe_balance_loss_backward(const void* logits, const float* share, const float* grad_loss, int64_t n_tokens,
+                               int32_t n_expert, int32_t dtype, float scale, void* grad_logits, fmoe_stream_t stream);
+
 /* ------------------------------------------------------------------------
  * Routing: counting, bucketing, capacity            (integer work, bit-exact)
  * ---------------------------------------------------------------------- */

@@ -155,3 +155,32 @@ def test_limit_and_prune(n, E, cap):
     assert (pruned.cpu().numpy() == want).all()
     assert (granted.cpu().numpy() == np.minimum(seen, cap)).all()
     assert (left.cpu().numpy() == cap - seen).all()
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("T,E", [(1, 2), (9, 16), (1500, 33), (40, 256), (300, 300)])
+def test_balance_loss(T, E, dtype):
+    """Value and logit gradient against the definition in fp64; 16-bit gradients are rounded once.  (300 experts: the
+    form in torch operators, which rounds the probabilities and their mean to the logits' type.)"""
+    from fastermoe_b200.gates.gshard_gate import balance_loss_top1
+    torch.manual_seed(T + E)
+    logits = torch.randn(T, E, device="cuda").to(dtype).requires_grad_(True)
+    idx = torch.randint(0, E, (T, 2), device="cuda")
+    loss = balance_loss_top1(idx[:, 0], logits, E, E)
+    grad, = torch.autograd.grad(3 * loss, logits, retain_graph=True)
+    ref = logits.detach().double().requires_grad_(True)
+    share = torch.bincount(idx[:, 0], minlength=E).double() / T
+    want = (share * torch.softmax(ref, 1).mean(0)).mean() * E ** 2
+    want_grad, = torch.autograd.grad(3 * want, ref, create_graph=True)
+    eps = torch.finfo(dtype).eps
+    rel = 1e-5 if E <= 256 else 4 * eps + 1e-5
+    assert loss.dtype == torch.float32 and abs(float(loss.detach()) - float(want.detach())) <= rel * float(want.detach())
+    floor = float(want_grad.abs().max())
+    if dtype == torch.float16:
+        floor += 6e-8 / eps             # fp16 subnormals
+    torch.testing.assert_close(grad.double(), want_grad.detach(), rtol=4 * eps + 1e-5, atol=(8 * eps + 1e-6) * floor)
+    if dtype == torch.float32:          # the gradient has a gradient
+        g, = torch.autograd.grad(loss, logits, create_graph=True)
+        w, = torch.autograd.grad(want, ref, create_graph=True)
+        torch.testing.assert_close(torch.autograd.grad((g * g).sum(), logits)[0].double(), torch.autograd.grad((w * w).sum(), ref)[0],
+                                   rtol=1e-3, atol=1e-5 * float(w.abs().max()) ** 2)
