@@ -79,7 +79,7 @@ def _shadow_plan(policy_fn, routing, experts, num_expert, world_size, d_model, f
     return stored, workers
 
 
-def _whole_layer(inp, gate, gate_score, expert_fn, experts):
+def _whole_layer(inp, gate, gate_score, expert_fn, experts, num_expert):
     """The layer as one library call (functions.MoeMlp), or None where somebody may look at or replace a step of it:
     a subclass or hook of the experts, another expert_fn, an operator profile, operands the kernels do not take."""
     operands = getattr(experts, "whole_layer_operands", None)
@@ -87,12 +87,12 @@ def _whole_layer(inp, gate, gate_score, expert_fn, experts):
             gate_score.numel() != gate.numel() or gate.dtype != torch.int64 or fmoe_cuda.profiling() or
             getattr(expert_fn, "__func__", None) is not FMoE.expert_fn):
         return None
-    found = operands(inp)
+    found = operands(inp, num_expert)
     if found is None:
         return None
     act, w1, b1, w2, b2 = found
     keep = torch.is_grad_enabled() and any(t is not None and t.requires_grad for t in (inp, gate_score, w1, b1, w2, b2))
-    return MoeMlp.apply(inp, gate, gate_score.reshape(gate.shape), w1, b1, w2, b2, act, keep)
+    return MoeMlp.apply(inp, gate.contiguous(), gate_score.reshape(gate.shape), w1, b1, w2, b2, act, keep)
 
 
 def _fmoe_general_global_forward(inp, gate, expert_fn, policy_fn, experts, num_expert, world_size,
@@ -108,7 +108,7 @@ def _fmoe_general_global_forward(inp, gate, expert_fn, policy_fn, experts, num_e
     the [T*k, d] tensor the reference returns.  Also returns ``stored_models``.
     """
     if world_size == 1 and fused and gate_score is not None:
-        out = _whole_layer(inp, gate, gate_score, expert_fn, experts)
+        out = _whole_layer(inp, gate, gate_score, expert_fn, experts, num_expert)
         if out is not None:
             return out, _no_shadow_flags(1, num_expert)
     top_k = gate.shape[1] if gate.dim() == 2 else 1

@@ -54,18 +54,19 @@ class _Expert(nn.Module):
             return _lib.ACT_SILU
         return code
 
-    def whole_layer_operands(self, inp):
+    def whole_layer_operands(self, inp, num_expert):
         """(activation code, w1, b1, w2, b2) when nothing can tell a call of forward() from the fused layer call on
-        the same parameters; else None."""
+        the same parameters; else None (parameters that do not fit together are left to the single operators' checks)."""
         if not _plain(self, _Expert) or torch.nn.modules.module._has_any_global_hook():
             return None
         code = self._kernel_code()
         up, down = self.htoh4, self.h4toh
         w1, b1, w2, b2 = up.weight, up.bias, down.weight, down.bias
-        if code is None or inp.dtype not in _KERNEL_DTYPES or inp.dim() != 2 or inp.shape[1] != w1.shape[2]:
+        if code is None or inp.dtype not in _KERNEL_DTYPES or inp.dim() != 2 or w1.dim() != 3:
             return None
-        for t in (w1, b1, w2, b2):
-            if t is not None and (t.dtype != inp.dtype or t.device != inp.device or not t.is_contiguous()):
+        d, h = inp.shape[1], w1.shape[1]
+        for t, shape in ((w1, (num_expert, h, d)), (b1, (num_expert, h)), (w2, (num_expert, d, h)), (b2, (num_expert, d))):
+            if t is not None and (t.shape != shape or t.dtype != inp.dtype or t.device != inp.device or not t.is_contiguous()):
                 return None
         return code, w1, b1, w2, b2
 

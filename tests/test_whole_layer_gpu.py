@@ -69,6 +69,15 @@ def test_partial_gradients():
     assert torch.equal(x.grad, want[1])
 
 
+def test_parameters_that_do_not_fit_are_refused():
+    """The fused call leaves them to the single operators, whose checks raise."""
+    for name, shape in (("htoh4", (4, 512, 264)), ("h4toh", (4, 256, 504)), ("htoh4", (3, 512, 256))):
+        m, x = make(20, 256, 512, 4, 2)
+        getattr(m.experts, name).weight = torch.nn.Parameter(torch.zeros(shape, device="cuda", dtype=torch.bfloat16))
+        with pytest.raises((AssertionError, RuntimeError)):
+            m(x)
+
+
 @pytest.mark.parametrize("act", ["gelu", "silu"])
 def test_hooks_are_called(act):
     m, x = make(20, 256, 512, 4, 2, act)
