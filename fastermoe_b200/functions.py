@@ -569,11 +569,18 @@ class FusedExpertMLP(Function):
     applied in the epilogue of the second layer's input-gradient GEMM."""
 
     @staticmethod
+    def _below_activation(ctx):
+        """A tensor on the input side of the activation (x, w1 or b1) needs a gradient, which takes the derivative.  (Asked
+        of the arguments as they came in: a contiguous copy made in forward() needs no gradient of its own.)"""
+        need = ctx.needs_input_grad
+        return need[0] or need[2] or need[3]
+
+    @staticmethod
     def forward(ctx, x, offsets, w1, b1, w2, b2, act, exch=None, keep=True):
         """``keep``: a backward may follow.  ``exch``: the PlannedExchange whose scatter produced ``x`` (and whose scatter of the output
         gradient will produce ``grad_y``); a pending arrival of it is waited for tile by tile."""
         x = x.contiguous()
-        want_pre = keep and act in _SAVES_DERIVATIVE and (x.requires_grad or w1.requires_grad)
+        want_pre = keep and act in _SAVES_DERIVATIVE and FusedExpertMLP._below_activation(ctx)
         arrival = exch.take_pending() if exch is not None else None
         h, pre = fmoe_cuda.linear_forward_act(x, offsets, w1, b1, act, want_pre=want_pre, arrival=arrival)
         y = x.new_empty((x.shape[0], w2.shape[1]))
@@ -594,6 +601,8 @@ class FusedExpertMLP(Function):
         if act == _lib.ACT_RELU:
             act_pre = h
         elif act in _SAVES_DERIVATIVE:
+            if pre is None and FusedExpertMLP._below_activation(ctx):
+                raise RuntimeError("FusedExpertMLP: the forward (keep=False) stored no activation derivative for this backward")
             act_pre = pre
         # The first layer's bias gradient is the column sum of gh: the input-gradient kernel of the
         # second layer returns it, so the first layer's backward does not read gh once more for it.

@@ -193,3 +193,56 @@ def test_balance_loss(T, E, dtype):
         w, = torch.autograd.grad(want, ref, create_graph=True)
         torch.testing.assert_close(torch.autograd.grad((g * g).sum(), logits)[0].double(), torch.autograd.grad((w * w).sum(), ref)[0],
                                    rtol=1e-3, atol=1e-5 * float(w.abs().max()) ** 2)
+
+
+def expert_gradients(m, x, idx, score, g, act):
+    """Gradients of the experts' parameters and of x, given the choice of experts and its weights, by autograd in fp64."""
+    fn = {"gelu": torch.nn.functional.gelu, "silu": torch.nn.functional.silu}[act]
+    p = {n: t.detach().double().requires_grad_(True) for n, t in m.experts.named_parameters()}
+    xr = x.detach().double().requires_grad_(True)
+    hid = fn(torch.einsum("ehd,td->teh", p["htoh4.weight"], xr) + p["htoh4.bias"])
+    y = torch.einsum("edh,teh->ted", p["h4toh.weight"], hid) + p["h4toh.bias"]
+    rows = torch.gather(y, 1, idx.unsqueeze(-1).expand(-1, -1, y.shape[2]))
+    (score.detach().double().unsqueeze(-1) * rows).sum(1).backward(g.double())
+    return {n: t.grad for n, t in p.items()}, xr.grad
+
+
+@pytest.mark.parametrize("form", ["one_call", "operators"])
+@pytest.mark.parametrize("act", ["gelu", "silu"])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("d,h", [(256, 320), (72, 200)])
+@pytest.mark.parametrize("trained", ["htoh4.bias", "htoh4.bias h4toh.weight h4toh.bias", "htoh4.weight", "h4toh.weight"])
+def test_some_parameters_trained(form, act, dtype, d, h, trained):
+    """Any subset of the experts' parameters may be trained while input and gate need no gradient: the first layer's bias
+    needs the activation's derivative as much as its weight does.  Bounds as in test_silu_against_fp32."""
+    m, x = make(90, d, h, 4, 2, act, dtype)
+    x.requires_grad_(False)
+    if form == "operators":
+        m.experts.register_forward_hook(lambda *a: None)
+    m.requires_grad_(False)
+    for n in trained.split():
+        m.experts.get_parameter(n).requires_grad_(True)
+    g = torch.randn(90, d, device="cuda").to(dtype)
+    idx, score = m.gate(x)
+    want, _ = expert_gradients(m, x, idx, score, g, act)
+    m(x).backward(g)
+    rel = 1e-5 if dtype == torch.float32 else 2e-2
+    for n, p in m.experts.named_parameters():
+        if n in trained.split():
+            assert float((p.grad.double() - want[n]).norm()) <= rel * float(want[n].norm()), n
+        else:
+            assert p.grad is None
+
+
+@pytest.mark.parametrize("act", ["gelu", "silu"])
+def test_input_gradient_of_strided_rows(act):
+    """A call of the experts on a transposed input, first layer frozen: its gradient passes the activation."""
+    m, x = make(40, 256, 320, 1, 1, act, torch.float32)
+    m.experts.htoh4.requires_grad_(False)
+    xt = x.detach().t().contiguous().t().requires_grad_(True)
+    out = m.experts(xt, torch.tensor([40]))
+    g = torch.randn_like(out)
+    out.backward(g)
+    one = torch.ones(40, 1, device="cuda")
+    _, want = expert_gradients(m, x, torch.zeros(40, 1, dtype=torch.int64, device="cuda"), one, g, act)
+    assert float((xt.grad.double() - want).norm()) <= 1e-5 * float(want.norm())
