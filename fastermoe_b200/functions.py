@@ -696,7 +696,11 @@ class GateTopK(Function):
 def gate_topk(logits, k, softmax=False):
     """Top-k over the last dimension with the library's kernel (CUDA tensors; k <= 8).  A CPU
     tensor, which no GPU code path produces, is answered by torch.topk.  Returns (values, indices);
-    ``softmax``: the values are the softmax over the selected logits."""
+    ``softmax``: the values are the softmax over the selected logits, in the logits' dtype, or in fp32 where
+    autocast forms softmaxes in fp32."""
+    if softmax and logits.is_cuda and logits.dtype != torch.float32 and torch.is_autocast_enabled("cuda"):
+        val, idx = gate_topk(logits, k)
+        return torch.softmax(val, dim=-1), idx
     if logits.is_cuda:
         if k > 8 or logits.dtype not in (torch.float32, torch.float16, torch.bfloat16):
             raise RuntimeError(f"gate_topk: k={k}, dtype={logits.dtype} is outside what the kernel takes "

@@ -246,3 +246,25 @@ def test_input_gradient_of_strided_rows(act):
     one = torch.ones(40, 1, device="cuda")
     _, want = expert_gradients(m, x, torch.zeros(40, 1, dtype=torch.int64, device="cuda"), one, g, act)
     assert float((xt.grad.double() - want).norm()) <= 1e-5 * float(want.norm())
+
+
+@pytest.mark.parametrize("param_dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("low", [torch.bfloat16, torch.float16])
+def test_gate_scores_under_autocast(low, param_dtype):
+    """Autocast forms softmaxes in fp32: the scores, their dtype and the gate's gradients are those of the softmax
+    operator on the selected logits, to the last bit."""
+    m, x = make(64, 256, 512, 8, 2, "gelu", param_dtype)
+    g = torch.randn(64, 2, device="cuda")
+    grads = []
+    for fused in (True, False):
+        m.zero_grad()
+        x.grad = None
+        with torch.autocast("cuda", low):
+            m.gate.softmax_scores = fused
+            idx, score = m.gate(x)
+            if not fused:
+                score = torch.nn.functional.softmax(score, dim=-1)
+        assert score.dtype == torch.float32
+        score.backward(g)
+        grads.append([idx, score.detach(), x.grad] + [p.grad for p in m.gate.parameters()])
+    assert all(torch.equal(a, b) for a, b in zip(*grads))
