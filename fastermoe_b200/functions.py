@@ -719,26 +719,19 @@ class BalanceLoss(Function):
     first choice is e and m_e the mean softmax probability of e, in fp32 with the library's kernels."""
 
     @staticmethod
-    def torch_form(logits, first_choice, scale):
-        share = torch.zeros(logits.shape[1], device=logits.device).scatter_add(
-            0, first_choice, torch.ones_like(first_choice, dtype=torch.float)) / logits.shape[0]
-        return (share * torch.softmax(logits.float(), dim=1).mean(dim=0)).sum() * scale
-
-    @staticmethod
     def forward(ctx, logits, first_choice, scale):
-        logits = logits.contiguous()
-        loss, share = fmoe_cuda.balance_loss(logits, first_choice, scale)
+        loss, share = fmoe_cuda.balance_loss(logits.contiguous(), first_choice, scale)
         ctx.scale = scale
-        ctx.save_for_backward(logits, first_choice, share)
+        ctx.save_for_backward(logits, share)
         return loss
 
     @staticmethod
     def backward(ctx, grad_loss):
-        logits, first_choice, share = ctx.saved_tensors
+        logits, share = ctx.saved_tensors
         if torch.is_grad_enabled() and (logits.requires_grad or grad_loss.requires_grad):     # a graph of this gradient is wanted
-            loss = BalanceLoss.torch_form(logits, first_choice, ctx.scale)
+            loss = (share * torch.softmax(logits.float(), dim=1).mean(dim=0)).sum() * ctx.scale
             return torch.autograd.grad(loss, logits, grad_loss, create_graph=True)[0], None, None
-        return fmoe_cuda.balance_loss_backward(logits, share, grad_loss.contiguous(), ctx.scale), None, None
+        return fmoe_cuda.balance_loss_backward(logits.contiguous(), share, grad_loss.contiguous(), ctx.scale), None, None
 
 
 class Slice(Function):

@@ -268,3 +268,26 @@ def test_gate_scores_under_autocast(low, param_dtype):
         score.backward(g)
         grads.append([idx, score.detach(), x.grad] + [p.grad for p in m.gate.parameters()])
     assert all(torch.equal(a, b) for a, b in zip(*grads))
+
+
+def test_balance_loss_keeps_its_graph():
+    """The second derivative reaches logits in any layout, and the choices may be overwritten after the call."""
+    from fastermoe_b200.gates.gshard_gate import balance_loss_top1
+    idx = torch.randint(0, 12, (30,), device="cuda")
+    plain = torch.randn(30, 12, device="cuda")
+    want = None
+    for strided in (False, True):
+        leaf = (plain.t().contiguous() if strided else plain.clone()).requires_grad_(True)
+        choice = idx.clone()
+        loss = balance_loss_top1(choice, leaf.t() if strided else leaf, 12, 12)
+        choice.zero_()
+        first, = torch.autograd.grad(loss, leaf, create_graph=True)
+        second, = torch.autograd.grad((first * first).sum(), leaf)
+        got = [t.detach().t() if strided else t.detach() for t in (first, second)]
+        if want is None:
+            ref = plain.double().requires_grad_(True)
+            share = torch.bincount(idx, minlength=12).double() / 30
+            g, = torch.autograd.grad((share * torch.softmax(ref, 1).mean(0)).sum() * 12, ref, create_graph=True)
+            want = [g.detach(), torch.autograd.grad((g * g).sum(), ref)[0]]
+        for a, w in zip(got, want):
+            torch.testing.assert_close(a.double(), w, rtol=1e-4, atol=1e-5 * float(w.abs().max()))
