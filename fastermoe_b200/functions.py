@@ -714,6 +714,13 @@ def gate_topk(logits, k, softmax=False):
     return (torch.softmax(val, dim=-1), idx) if softmax else (val, idx)
 
 
+def plain_autograd():
+    """True when operators are run eagerly under reverse-mode autograd alone.  Tracers, function transforms (vmap, jvp,
+    grad) and forward-mode levels see through torch operators, but have no rule for a Function of the library."""
+    return not (torch.compiler.is_compiling() or torch.jit.is_tracing() or torch._C._are_functorch_transforms_active() or
+                torch.autograd.forward_ad._current_level >= 0)
+
+
 class BalanceLoss(Function):
     """scale * sum_e c_e m_e of the capacity gates (fmoe/gates/gshard_gate.py:27-35), c_e the share of the tokens whose
     first choice is e and m_e the mean softmax probability of e, in fp32 with the library's kernels."""

@@ -5,16 +5,17 @@ import torch
 import torch.nn.functional as F
 
 from .. import fmoe_cuda
-from ..functions import BalanceLoss
+from ..functions import BalanceLoss, plain_autograd
 from .naive_gate import NaiveGate
 from .utils import limit_by_capacity
 
 
 def balance_loss_top1(top1_idx, gate_score, tot_expert, num_expert):
     """mean(fraction routed * mean softmax prob) * num_expert^2 (gshard_gate.py:27-35)."""
-    if (gate_score.is_cuda and gate_score.dim() == 2 and gate_score.shape[0] > 0 and
+    if (plain_autograd() and gate_score.is_cuda and gate_score.dim() == 2 and gate_score.shape[0] > 0 and
             tot_expert == gate_score.shape[1] <= fmoe_cuda.BALANCE_MAX_EXPERTS and
-            gate_score.dtype in (torch.float32, torch.float16, torch.bfloat16) and top1_idx.dtype == torch.int64):
+            gate_score.dtype in (torch.float32, torch.float16, torch.bfloat16) and
+            top1_idx.dtype == torch.int64 and top1_idx.device == gate_score.device and top1_idx.shape == gate_score.shape[:1]):
         return BalanceLoss.apply(gate_score, top1_idx, num_expert ** 2 / tot_expert)
     S = gate_score.shape[0]
     c_e = torch.scatter_add(torch.zeros(tot_expert, device=top1_idx.device), 0, top1_idx,

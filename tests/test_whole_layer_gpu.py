@@ -291,3 +291,36 @@ def test_balance_loss_keeps_its_graph():
             want = [g.detach(), torch.autograd.grad((g * g).sum(), ref)[0]]
         for a, w in zip(got, want):
             torch.testing.assert_close(a.double(), w, rtol=1e-4, atol=1e-5 * float(w.abs().max()))
+
+
+def test_balance_loss_of_calls_left_to_torch():
+    """Function transforms, forward mode, tracing and compilation see the loss as operators, and a call may count fewer
+    choices than there are logits: the same values as the operators give in fp64."""
+    from fastermoe_b200.gates.gshard_gate import balance_loss_top1
+    import torch.autograd.forward_ad as fa
+    idx = torch.randint(0, 12, (30,), device="cuda")
+    logits = torch.randn(30, 12, device="cuda")
+    tangent = torch.randn_like(logits)
+
+    def loss(v, choice=idx):
+        return balance_loss_top1(choice, v, 12, 12)
+
+    def want(v, choice=idx):
+        return (torch.bincount(choice, minlength=12).double() / 30 * torch.softmax(v, 1).mean(0)).sum() * 12
+
+    def close(a, b):
+        torch.testing.assert_close(a.double(), b.double(), rtol=1e-5, atol=1e-6)
+
+    ref = logits.double().requires_grad_(True)
+    grad, = torch.autograd.grad(want(ref), ref)
+    slope = (grad * tangent.double()).sum()
+    value, along = torch.func.jvp(loss, (logits,), (tangent,))
+    close(value, want(logits.double()))
+    close(along, slope)
+    close(torch.func.grad(loss)(logits), grad)
+    close(torch.func.vmap(loss)(torch.stack([logits, 2 * logits])), torch.stack([want(s * logits.double()) for s in (1, 2)]))
+    with fa.dual_level():
+        close(fa.unpack_dual(loss(fa.make_dual(logits, tangent))).tangent, slope)
+    close(torch.jit.trace(loss, (logits,))(2 * logits), want(2 * logits.double()))
+    close(torch.compile(loss, backend="eager", fullgraph=True)(logits), want(logits.double()))
+    close(loss(logits, idx[:20]), want(logits.double(), idx[:20]))
