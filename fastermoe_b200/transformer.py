@@ -46,10 +46,12 @@ class _Expert(nn.Module):
 
     def _kernel_code(self):
         """Code of the activation that the products' epilogues apply, or None.  SiLU is among them as long as the
-        three modules are called by nobody's hook: each is a call of its own otherwise."""
+        three modules are called by nobody's hook and the weights lie as the kernels read them: each is a call of its
+        own otherwise (which copies a strided weight)."""
         code = activation_code(self.activation)
         if code is None and (self.activation is F.silu or _plain(self.activation, nn.SiLU)) and \
                 _plain(self.htoh4, FMoELinear) and _plain(self.h4toh, FMoELinear) and \
+                self.htoh4.weight.is_contiguous() and self.h4toh.weight.is_contiguous() and \
                 not torch.nn.modules.module._has_any_global_hook():
             return _lib.ACT_SILU
         return code

@@ -324,3 +324,17 @@ def test_balance_loss_of_calls_left_to_torch():
     close(torch.jit.trace(loss, (logits,))(2 * logits), want(2 * logits.double()))
     close(torch.compile(loss, backend="eager", fullgraph=True)(logits), want(logits.double()))
     close(loss(logits, idx[:20]), want(logits.double(), idx[:20]))
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_silu_with_a_strided_weight(dtype):
+    """A SiLU layer takes a transposed weight (its linears copy it): same output and gradients as with the copy, up to
+    the activation's rounding where it is an operator of its own."""
+    m, x = make(20, 256, 512, 4, 2, "silu", dtype)
+    g = torch.randn(20, 256, device="cuda").to(dtype)
+    want = step(m, x, g)
+    for lin in (m.experts.htoh4, m.experts.h4toh):
+        lin.weight = torch.nn.Parameter(lin.weight.detach().transpose(1, 2).contiguous().transpose(1, 2))
+    tol = 1e-5 if dtype == torch.float32 else 2e-2
+    for a, b in zip(step(m, x, g), want):
+        assert float((a.double() - b.double()).norm()) <= tol * float(b.double().norm())
