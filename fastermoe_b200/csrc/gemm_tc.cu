@@ -1795,6 +1795,11 @@ bool tc_forward_supported(const LinearArgs& a) {
 }
 
 bool tc_backward_supported(const LinearBwdArgs& a) {
+    // Off the 64-element grid, column sums may come without a scratch buffer (or to an odd address): the FFMA kernels
+    // need neither.
+    if (a.grad_x_colsum && !tc_grid_widths(a.in_feat, a.out_feat) &&
+        (!a.scratch || !aligned16(a.scratch) || ((uintptr_t)a.grad_x_colsum & 3)))
+        return false;
     return shape_ok(a.n_rows, a.in_feat, a.out_feat, a.n_expert, a.dtype) && aligned16(a.grad_y) &&
            aligned16(a.weight) && (!a.x || aligned16(a.x)) && (!a.grad_x || aligned16(a.grad_x)) &&
            (!a.grad_w || aligned16(a.grad_w)) && (!a.act_pre || aligned16(a.act_pre)) &&

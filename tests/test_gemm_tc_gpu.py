@@ -394,3 +394,29 @@ def test_token_minor_epilogues(fc, act):
         g = gy[p:p + c].float() @ w[e].float()
         close(gx[p:p + c], g * (saved[p:p + c].float() > 0) if act == "relu" else g)
         p += c
+
+
+@pytest.mark.parametrize("what", ["no_scratch", "odd_address"])
+@pytest.mark.parametrize("fin,fout", [(200, 136), (64, 64), (30, 50)])
+def test_column_sums_without_scratch(what, fin, fout):
+    """Off the 64-element grid the column sums need neither the scratch buffer nor an even number of elements before them."""
+    from fastermoe_b200 import _lib
+    counts = [17, 0, 23]
+    B, E = sum(counts), len(counts)
+    x, gy = torch.randn(B, fin, device="cuda").bfloat16(), torch.randn(B, fout, device="cuda").bfloat16()
+    w = (torch.randn(E, fout, fin, device="cuda") / np.sqrt(fout)).bfloat16()
+    off = torch.tensor([0, 17, 17, 40], device="cuda")
+    gx, gw = torch.empty_like(x), torch.empty_like(w)
+    cs = torch.empty(E * fin + 1, device="cuda", dtype=torch.bfloat16)[int(what == "odd_address"):]
+    nbytes = _lib.lib.fmoe_linear_scratch_bytes(B, fin, fout, E, _lib.BF16)
+    scratch = None if what == "no_scratch" else torch.empty(nbytes, dtype=torch.uint8, device="cuda")
+    ptr = [None if t is None else t.data_ptr() for t in (gy, x, w, off, None, gx, gw, None, cs)]
+    rc = _lib.lib.fmoe_linear_backward_colsum(*ptr, B, fin, fout, E, _lib.BF16, _lib.ACT_NONE, 0,
+                                              None if scratch is None else scratch.data_ptr(), None)
+    assert rc == 0, _lib.lib.fmoe_last_error_string()
+    torch.cuda.synchronize()
+    p = 0
+    for e, c in enumerate(counts):
+        close(gx[p:p + c], gy[p:p + c].float() @ w[e].float())
+        close(cs[e * fin:(e + 1) * fin], gx[p:p + c].float().sum(0))
+        p += c
