@@ -1532,7 +1532,8 @@ bool use_pairs(int mode, int64_t n_rows, int n_expert, int64_t n_out) {
 struct Form { bool swap, pair; int tile_n; };
 Form pick_form(int mode, int64_t n_rows, int n_expert, int64_t n_out, int64_t n_contr) {
     if (tc_grid_widths(n_contr, n_out)) return Form{false, use_pairs(mode, n_rows, n_expert, n_out), 0};
-    const bool pair = n_rows > (int64_t)32 * n_expert;
+    const int form = forced_form();
+    const bool pair = form == FMOE_GEMM_PAIR || (form != FMOE_GEMM_SINGLE && n_rows > (int64_t)32 * n_expert);
     return Form{true, pair, pair ? 256 : 64};
 }
 // CTAs the persistent GEMM grids may use: all SMs, or fewer (FMOE_B200_GEMM_SMS=n, or

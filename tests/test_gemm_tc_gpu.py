@@ -318,10 +318,9 @@ def test_input_gradient_column_sums(fc, dtype, form):
 
 
 TOKEN_MINOR = [
-    # few tokens per expert (one CTA per tile): edges of the 32-token steps, experts without any
+    # on the 64-element grid: the token-major kernels at the same row counts
     ([1, 31, 32, 33, 0, 63, 64, 65], 256, 384),
     ([3, 0, 0, 1], 2048, 1024),
-    # pairs of CTAs: edges of the 64-token steps and of the 256-token tiles
     ([255, 256, 257, 0, 1, 129], 512, 256),
     ([700, 37], 256, 832),
     # widths off the 64-element grid, the smallest ones, columns that end inside a 32-column block
@@ -420,3 +419,34 @@ def test_column_sums_without_scratch(what, fin, fout):
         close(gx[p:p + c], gy[p:p + c].float() @ w[e].float())
         close(cs[e * fin:(e + 1) * fin], gx[p:p + c].float().sum(0))
         p += c
+
+
+def gemm_kernels(call):
+    """Template arguments (mode, bf16, pair, token-minor) of the tensor-core products that ``call`` launches."""
+    import re
+    call()
+    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as prof:
+        call()
+        torch.cuda.synchronize()
+    found = []
+    for e in prof.events():
+        m = re.search(r"grouped_gemm_kernel<([^>]*)>", e.name)
+        if m:
+            words = re.sub(r"\((int|bool)\)", "", m.group(1)).replace("true", "1").replace("false", "0")
+            found.append(tuple(int(w) for w in words.split(",")))
+    return found
+
+
+def test_forced_form_off_the_grid(fc):
+    """"pair" and "tc1" force the form of widths off the 64-element grid too; "auto" goes by the rows per expert."""
+    from fastermoe_b200 import _lib
+    fin, fout = 200, 136
+    w = torch.randn(2, fout, fin, device="cuda").bfloat16()
+    for rows, auto in ((20, 0), (400, 1)):
+        x = torch.randn(rows, fin, device="cuda").bfloat16()
+        off = torch.tensor([0, rows // 2, rows], device="cuda")
+        for form, pair in (("auto", auto), ("pair", 1), ("tc1", 0)):
+            fc.set_gemm_form(form)
+            ran = gemm_kernels(lambda: (fc.linear_forward_act(x, off, w, None, _lib.ACT_NONE),
+                                        fc.linear_backward_act(x.new_ones(rows, fout), x, off, w, None, _lib.ACT_NONE)))
+            assert sorted(ran)[:2] == [(0, 1, pair, 1), (1, 1, pair, 1)], (form, rows, ran)
