@@ -757,7 +757,8 @@ def run_ours(args):
         step_resident()
     dur = tprof.durations_ms()
     fmoe_cuda.set_profile(None)
-    # kernels of this library launched per step (counted on an eager step; a replayed graph runs the same ones)
+    # kernels of this library launched per step (counted on an eager step, whose layer a profile runs operator by operator;
+    # the one call per direction of an unprofiled layer and a replayed graph run the same kernels)
     prof = fmoe_cuda.Profile()
     fmoe_cuda.set_profile(prof)
     step_resident()

@@ -30,9 +30,11 @@ from ._lib import lib, check
 _DT = {torch.float32: _lib.F32, torch.float16: _lib.F16, torch.bfloat16: _lib.BF16}
 
 
-# Kernel launches issued by one call of each C entry point (for launch accounting).
+# Kernel launches issued by one call of each C entry point (for launch accounting; the bucketing ones issue one instead
+# of four for few entries).
 _KERNELS = {"expert_count": 1, "assign_pos": 4, "count_and_pos": 4, "limit_by_capacity": 1,
-            "prune_gate_by_capacity": 4, "local_scatter": 1, "local_gather": 3, "local_gather_inv": 1,
+            "prune_gate_by_capacity": 4, "limit_and_prune": 4, "balance_loss": 2, "local_scatter": 1, "local_gather": 3,
+            "local_gather_inv": 1,
             "local_gather_sum": 1, "local_gather_add": 3, "combine_forward": 1, "combine_backward": 1, "linear_forward": 1,
             "linear_backward": 3, "expert_exchange": 2, "generate_cached_count": 1,
             "peer_scatter": 2, "peer_gather": 2, "peer_plan": 1}
@@ -980,7 +982,7 @@ def combine_backward(grad_out, buf, inv, score, need_score_grad=True, need_buf_g
 
 def linear_forward_act(x, seg_offsets, weight, bias, activation, want_pre=False, arrival=None, departure=None, out=None):
     """Grouped GEMM with fused bias and activation.  Returns (y, act_deriv or None);
-    ``act_deriv`` (with ``want_pre`` and GELU) holds gelu'(pre-activation), the factor
+    ``act_deriv`` (with ``want_pre`` and GELU or SiLU) holds the derivative at the pre-activation, the factor
     that linear_backward_act multiplies into the input gradient.  ``arrival``: a PendingArrival
     whose exchange is still filling ``x``; the call closes it.  ``departure``: a PendingArrival of
     peer_gather_planned_async that forwards ``out`` (the preallocated y) while the product runs; the
@@ -1013,7 +1015,7 @@ def linear_backward_act(grad_y, x, seg_offsets, weight, act_pre, activation, nee
                         arrival=None, departure=None, grad_x=None):
     """Grouped GEMM backward.  ``act_pre`` (shape of x) fuses the backward of the
     activation that produced ``x`` into the input gradient: for ReLU pass the activation
-    output, for GELU the derivative buffer of linear_forward_act.  Returns (dX, dW, db), and with
+    output, for GELU and SiLU the derivative buffer of linear_forward_act.  Returns (dX, dW, db), and with
     ``want_gx_colsum`` a fourth tensor [E, in_feat]: the per-expert column sums of dX (the bias
     gradient of the layer that produced ``x``), which the input-gradient kernel computes on the way."""
     _check_cuda(grad_y, x, seg_offsets, weight, act_pre)

@@ -280,7 +280,7 @@ size_t fmoe_linear_scratch_bytes(int64_t n_rows, int64_t in_feat, int64_t out_fe
  * fmoe/transformer.py:28).  X [n_rows,in_feat], W [E,out_feat,in_feat],
  * bias [E,out_feat] or NULL, Y [n_rows,out_feat], all row-major, dtype as given;
  * accumulation is fp32.  seg_offsets: DEVICE int64[E+1], exclusive prefix sum
- * of the reference's expert_count.  pre_act (may be NULL; used with GELU):
+ * of the reference's expert_count.  pre_act (may be NULL; used with GELU and SiLU):
  * receives activation'(z) of the value z before the activation, in the tensor
  * dtype -- the factor the backward of the activation multiplies by, computed
  * here where z is still in registers. */
