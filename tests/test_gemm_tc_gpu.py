@@ -450,3 +450,58 @@ def test_forced_form_off_the_grid(fc):
             ran = gemm_kernels(lambda: (fc.linear_forward_act(x, off, w, None, _lib.ACT_NONE),
                                         fc.linear_backward_act(x.new_ones(rows, fout), x, off, w, None, _lib.ACT_NONE)))
             assert sorted(ran)[:2] == [(0, 1, pair, 1), (1, 1, pair, 1)], (form, rows, ran)
+
+
+TOKEN_MINOR_EDGES = [
+    # the 32-token steps of one CTA and its 64-token tiles; widths with a column block of 8 and of 24
+    ([1, 31, 32, 33, 0, 63, 64, 65], 264, 200),
+    # the 64-token steps of a pair; its second CTA has 8 columns of 392 and none of 520
+    ([127, 128, 129, 191, 192, 193], 392, 520),
+    # segments that end on a 256-token tile, one before and one after it
+    ([255, 256, 257, 0, 1, 512], 136, 328),
+    ([700, 37], 72, 264),
+    ([3, 0, 0, 1], 2056, 1032),
+    ([5, 70], 32, 40),
+]
+
+
+@pytest.mark.parametrize("form", ["pair", "tc1"])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("counts,fin,fout", TOKEN_MINOR_EDGES)
+def test_token_minor_edges(fc, form, dtype, counts, fin, fout):
+    """Both forms of the products off the 64-element grid at the edges of their steps and tiles."""
+    fc.set_gemm_form(form)
+    test_token_minor_products(fc, dtype, counts, fin, fout)
+
+
+@pytest.mark.parametrize("form", ["pair", "tc1"])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("act", ["relu", "none", "gelu", "silu"])
+def test_token_minor_activations(fc, form, dtype, act):
+    """Every activation in both forms: value and saved derivative forward, the saved factor backward, against fp32."""
+    from fastermoe_b200 import _lib
+    fc.set_gemm_form(form)
+    code = {"relu": _lib.ACT_RELU, "none": _lib.ACT_NONE, "gelu": _lib.ACT_GELU, "silu": _lib.ACT_SILU}[act]
+    fn = {"relu": torch.relu, "none": lambda z: z * 1, "gelu": torch.nn.functional.gelu, "silu": torch.nn.functional.silu}[act]
+    counts, fin, fout = [40, 0, 97, 256, 5], 328, 200
+    E, B = len(counts), sum(counts)
+    x, gy = torch.randn(B, fin, device="cuda").to(dtype), torch.randn(B, fout, device="cuda").to(dtype)
+    w = ((torch.rand(E, fout, fin, device="cuda") * 2 - 1) / np.sqrt(fin)).to(dtype)
+    b = (torch.randn(E, fout, device="cuda") * 4).to(dtype)
+    saved = (torch.randn(B, fin, device="cuda").relu() if act == "relu" else torch.randn(B, fin, device="cuda")).to(dtype)
+    off = torch.tensor(np.concatenate([[0], np.cumsum(counts)]), dtype=torch.int64, device="cuda")
+    saves = act in ("gelu", "silu")
+    y, pre = fc.linear_forward_act(x, off, w, b, code, want_pre=saves)
+    alone, _ = fc.linear_forward_act(x, off, w, b, code)
+    assert torch.equal(y, alone)                       # the value does not depend on whether the derivative is kept
+    gx, _, _ = fc.linear_backward_act(gy, x, off, w, None if act == "none" else saved, code)
+    factor = {"relu": (saved > 0).float(), "none": torch.ones_like(saved).float()}.get(act, saved.float())
+    assert device_status() == 0
+    p = 0
+    for e, c in enumerate(counts):
+        z = (x[p:p + c].float() @ w[e].float().t() + b[e].float()).requires_grad_(True)
+        close(y[p:p + c], fn(z).detach())
+        if saves and c:
+            close(pre[p:p + c], torch.autograd.grad(fn(z).sum(), z)[0])
+        close(gx[p:p + c], gy[p:p + c].float() @ w[e].float() * factor[p:p + c])
+        p += c
