@@ -9,6 +9,7 @@
 #include "common.cuh"
 #include "gemm.h"
 #include <initializer_list>
+#include <type_traits>
 
 namespace fmoe {
 namespace {
@@ -19,34 +20,39 @@ namespace {
 // multiply-adds go out two columns at a time (fma.rn.f32x2), which leaves issue slots for those loads.  Each
 // output is still one fused multiply-add chain in ascending order of the contraction index.  Global loads of
 // the next 16 contraction steps are in registers while the current ones are multiplied; two shared-memory
-// buffers, one barrier per step.  Measured (4096 rows, 512 x 2048, fp32): 425 us with 4 x 4 micro-tiles, 216 now
-// (40 TFLOP/s; the FMA pipe is busy 69 % of the active cycles, the rest is the last wave and the latency of the
+// buffers, one barrier per step.  Measured (4096 rows, 512 x 2048, fp32): 425 us with 4 x 4 micro-tiles, 203 now
+// (42 TFLOP/s; the FMA pipe is busy 69 % of the active cycles, the rest is the last wave and the latency of the
 // operand loads).  Steps of 8 instead of 16 were slower (230 us): the loads then have too little time to arrive.
 constexpr int BN = 128, BK = 16;
 constexpr int SEG_CHUNK = 128;      // segment offsets looked at per round by find_tile
 
+// Four consecutive elements as they lie in memory, the ones past `valid` zero: one vector (VEC: 4 divides the extent, so
+// a vector is either inside or outside) or element by element.
 template <typename T, bool VEC>
-__device__ __forceinline__ void load4(const T* __restrict__ src, int valid, float* out) {
-    if (VEC) {
-        // (4 divides the extent: a vector is either inside or outside)
-        if (valid > 0) {
-            if (sizeof(T) == 4) {
-                const float4 q = __ldg(reinterpret_cast<const float4*>(src));
-                out[0] = q.x; out[1] = q.y; out[2] = q.z; out[3] = q.w;
-            } else {
-                const uint2 q = __ldg(reinterpret_cast<const uint2*>(src));
-                const T* h = reinterpret_cast<const T*>(&q);
-#pragma unroll
-                for (int i = 0; i < 4; ++i) out[i] = to_float<T>(h[i]);
-            }
+struct Raw4 {
+    using Word = typename std::conditional<sizeof(T) == 4, float, unsigned short>::type;
+    using Vec = typename std::conditional<sizeof(T) == 4, float4, uint2>::type;
+    typename std::conditional<VEC, Vec, Word[4]>::type q;
+    __device__ __forceinline__ void load(const T* __restrict__ src, int valid) {
+        if constexpr (VEC) {
+            q = valid > 0 ? __ldg(reinterpret_cast<const Vec*>(src)) : Vec{};
         } else {
 #pragma unroll
-            for (int i = 0; i < 4; ++i) out[i] = 0.f;
+            for (int i = 0; i < 4; ++i) q[i] = i < valid ? __ldg(reinterpret_cast<const Word*>(src) + i) : Word(0);
         }
-    } else {
-#pragma unroll
-        for (int i = 0; i < 4; ++i) out[i] = i < valid ? to_float<T>(src[i]) : 0.f;
     }
+    __device__ __forceinline__ void get(float* out) const {
+        const T* v = reinterpret_cast<const T*>(&q);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) out[i] = to_float<T>(v[i]);
+    }
+};
+
+template <typename T, bool VEC>
+__device__ __forceinline__ void load4(const T* __restrict__ src, int valid, float* out) {
+    Raw4<T, VEC> r;
+    r.load(src, valid);
+    r.get(out);
 }
 
 template <typename T, bool VEC>
@@ -69,24 +75,26 @@ __device__ __forceinline__ void store4(T* __restrict__ dst, int valid, const flo
     }
 }
 
-// One operand tile, R rows x BK contraction steps, staged in registers (stage) and then stored as sm[k][r].
+// One operand tile, R rows x BK contraction steps, staged in registers as it lies in memory and then stored in fp32 as
+// sm[k][r].  (Converting 16-bit elements when they are staged would wait for the loads before the multiply-adds that
+// should cover them.)
 // KC: the contraction index is contiguous in memory (element (r, k) at r * ld + k); otherwise the row index is
 // (element at k * ld + r).  rows / steps bound the tile: elements outside are zero.
 template <typename T, int R, int TH, bool KC, bool VEC>
 struct Operand {
     static constexpr int NV = R * BK / 4 / TH;      // vectors of four per thread
     static constexpr int LD = R + 4;
-    float stage[NV][4];
+    Raw4<T, VEC> stage[NV];
     __device__ __forceinline__ void load(const T* __restrict__ src, int64_t ld, int rows, int steps) {
 #pragma unroll
         for (int i = 0; i < NV; ++i) {
             const int v = threadIdx.x + i * TH;
             if (KC) {
                 const int r = v / (BK / 4), k = (v % (BK / 4)) * 4;
-                load4<T, VEC>(src + (int64_t)r * ld + k, r < rows ? steps - k : 0, stage[i]);
+                stage[i].load(src + (int64_t)r * ld + k, r < rows ? steps - k : 0);
             } else {
                 const int k = v / (R / 4), r = (v % (R / 4)) * 4;
-                load4<T, VEC>(src + (int64_t)k * ld + r, k < steps ? rows - r : 0, stage[i]);
+                stage[i].load(src + (int64_t)k * ld + r, k < steps ? rows - r : 0);
             }
         }
     }
@@ -94,13 +102,15 @@ struct Operand {
 #pragma unroll
         for (int i = 0; i < NV; ++i) {
             const int v = threadIdx.x + i * TH;
+            float f[4];
+            stage[i].get(f);
             if (KC) {
                 const int r = v / (BK / 4), k = (v % (BK / 4)) * 4;
 #pragma unroll
-                for (int j = 0; j < 4; ++j) sm[k + j][r] = stage[i][j];
+                for (int j = 0; j < 4; ++j) sm[k + j][r] = f[j];
             } else {
                 const int k = v / (R / 4), r = (v % (R / 4)) * 4;
-                *reinterpret_cast<float4*>(&sm[k][r]) = make_float4(stage[i][0], stage[i][1], stage[i][2], stage[i][3]);
+                *reinterpret_cast<float4*>(&sm[k][r]) = make_float4(f[0], f[1], f[2], f[3]);
             }
         }
     }
@@ -249,13 +259,20 @@ rows_gemm_kernel(const T* __restrict__ a, const T* __restrict__ w, const T* __re
     f32x2 acc[8][4];
     // B(k, n): MODE 0 -> W[n0+n, k] (k contiguous); MODE 1 -> W[k, n0+n] (n contiguous); rows of in_feat elements either way
     B::run(sm, a + tm.row0 * kdim, kdim, tm.rows, MODE == 0 ? wp + n0 * in_feat : wp + n0, in_feat, n_valid, kdim, acc);
-#pragma unroll
+    // One copy of the epilogue for the eight rows of a thread, which take their turn in acc[0].  (Unrolled, 64 copies of
+    // erff and of the derivative's expf are fetched by a block that runs each once: 128 rows of two experts, 64 x 256,
+    // fp32 took 45 us, 18 here; 4096 rows of four, 512 x 2048: 239 and 221.)
+#pragma unroll 1
     for (int i = 0; i < 8; ++i) {
         const int r = (i >> 2) * (BM / 2) + B::ty() * 4 + (i & 3);
-        if (r >= tm.rows) continue;
         const int64_t row = (tm.row0 + r) * ndim;
         float v[8];
-        unpair(acc[i], v);
+        unpair(acc[0], v);
+#pragma unroll
+        for (int u = 0; u < 7; ++u)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) acc[u][j] = acc[u + 1][j];
+        if (r >= tm.rows) continue;
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
             const int cidx = h * (BN / 2) + B::tx() * 4, valid = n_valid - cidx;
