@@ -1527,8 +1527,16 @@ bool use_pairs(int mode, int64_t n_rows, int n_expert, int64_t n_out) {
 // off the 64-element grid run on the tensor cores at all; on the grid it is the slower one (16384 rows of 32 skewed
 // experts, 2048 x 8192: 536 us token-major, 613 token-minor; 184 rows of 13: 75 and 83), so widths alone decide.
 // Off the grid, 3998 rows of six experts, 200 x 712: six products took 460 us on the FFMA pipe, 76 here.
+// The stored values of GELU and its derivative off the grid are gelu_pair's, not erff's as on the FFMA pipe; rounded to
+// bf16 both are equally far from GELU everywhere, rounded to fp16 the worst relative error is 1.4e-3 instead of 8e-4 for
+// arguments between -4 and -3 and the same elsewhere (computed over [-8, 8]).
 // tile_n: 64 tokens leave eight stages for streaming weights when experts have few rows; above 32 rows on average
-// pairs with 256 tokens, which pull fewer operand bytes per flop.
+// pairs with 256 tokens, which pull fewer operand bytes per flop.  Forward with GELU, us, one CTA / pairs, eight experts:
+//   rows per expert      32           64           128           256           512
+//   200 x 712        13.3/13.3    13.3/15.4     15.3/15.4     17.4/17.3     19.4/19.5
+//   1000 x 2000      21.5/21.4    21.5/21.5     27.6/23.6     37.9/25.6     59.5/33.8
+//   2056 x 4104      44.0/44.1    46.1/46.1     66.4/46.1    113.6/52.2    199.7/84.8
+// (4 rows: 13.3/13.2, 19.5/19.5, 42.0/44.0).  Up to the line the forms are within one tick of the clock, 2 us, of each other.
 struct Form { bool swap, pair; int tile_n; };
 Form pick_form(int mode, int64_t n_rows, int n_expert, int64_t n_out, int64_t n_contr) {
     if (tc_grid_widths(n_contr, n_out)) return Form{false, use_pairs(mode, n_rows, n_expert, n_out), 0};
