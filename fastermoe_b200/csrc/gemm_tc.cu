@@ -1631,12 +1631,11 @@ bool shape_ok(int64_t n_rows, int64_t in_feat, int64_t out_feat, int n_expert, i
            (int64_t)n_expert * out_feat < ((int64_t)1 << 31);
 }
 
-// Column sums of dY per expert segment (bias gradient), fp32 accumulate.  A cluster of kBiasSplit blocks per
+// Column sums of dY per expert segment (bias gradient), fp32 accumulate.  A cluster of gridDim.z blocks (bias_split) per
 // (128 columns, expert): each block sums a share of the segment's rows (16 column lanes of one 16-byte load each x 16
 // row lanes, four rows in flight per thread), the first one adds the shares, read through distributed shared memory, in
-// order.  One block per expert was bound by the longest segment: 16384 rows of 32 skewed experts, 2048 columns, took
-// 256 us, 32 now.
-constexpr int kBiasSplit = 8;
+// order.  Without the split the longest segment bounds the kernel.
+constexpr int kBiasSplitMax = 8;
 
 template <bool BF16>
 __global__ void __launch_bounds__(256)
@@ -1652,7 +1651,8 @@ bias_grad_tc_kernel(const uint16_t* __restrict__ dy, const int64_t* __restrict__
     const int col = blockIdx.x * COLS + cl * 8;
     int64_t lo, hi;
     safe_seg_range(seg, hs, e, n_rows, lo, hi);
-    const int64_t per = (hi - lo + kBiasSplit - 1) / kBiasSplit;
+    const int split = (int)gridDim.z;
+    const int64_t per = (hi - lo + split - 1) / split;
     const int64_t my_lo = lo + blockIdx.z * per, my_hi = min(hi, my_lo + per);
     float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
     if (col < out_feat) {
@@ -1695,9 +1695,11 @@ bias_grad_tc_kernel(const uint16_t* __restrict__ dy, const int64_t* __restrict__
     if (blockIdx.z == 0 && threadIdx.x < COLS) {
         const int c = blockIdx.x * COLS + threadIdx.x;
         if (c < out_feat) {
-            float t = 0.f;
+            float t = 0.f, part[kBiasSplitMax];
 #pragma unroll
-            for (int r = 0; r < kBiasSplit; ++r) t += *cluster.map_shared_rank(share + threadIdx.x, r);
+            for (int r = 0; r < kBiasSplitMax; ++r) part[r] = r < split ? *cluster.map_shared_rank(share + threadIdx.x, r) : 0.f;
+#pragma unroll
+            for (int r = 0; r < kBiasSplitMax; ++r) t += part[r];
             uint16_t* o = db + (size_t)e * out_feat + c;
             if (accumulate) t += cvt_in<BF16>(*o);
             const uint32_t packed = cvt_pack<BF16>(t, 0.f);
@@ -1780,17 +1782,39 @@ colsum_finish_kernel(const float* __restrict__ partial, const int64_t* __restric
     *o = cvt_pack<BF16>(t0, t1);
 }
 
+// Blocks per (128 columns, expert) of the bias gradient.  Up to a grid of 512 blocks a split costs nothing and shortens the
+// longest segment; past that, only when the average segment gives each block 64 rows, and up to 2048 blocks (1024 for
+// eighths of segments of less than 2048 rows): blocks without rows to speak of queue up in front of the products.
+// Whole backward with 1, 2, 4, 8 blocks, us (the kernel beside the products):
+//   experts x columns, rows each                    uniform              popularity 1 / (rank + 1)^1.2
+//    8 x 1024, 4096 (64 blocks unsplit)        119  105  103   92           209  166  139  135
+//   32 x 1024, 1024 (256)                      105   92   96  101           174  141  131  144
+//   64 x 1024,  512 (512)                      107  107  109  121           178  172  150  168
+//   32 x 4096,  512 (1024)                     277  279  289  328           408  324  326  353
+//   64 x 4096,  128 (2048)                     250  258  285  330           289  293  318  365
+int bias_split(int64_t n_rows, int n_expert, int64_t out_feat) {
+    const int64_t blocks = ceil_div(out_feat, 128) * n_expert, rows = n_rows / n_expert;
+    int split = 1;
+    while (split < kBiasSplitMax) {
+        const int64_t grid = 2 * split * blocks, most = split < 4 || rows >= 2048 ? 2048 : 1024;
+        if (grid > 512 && (grid > most || rows < 128 * split)) break;
+        split *= 2;
+    }
+    return split;
+}
+
 template <bool BF16>
 int launch_bias_grad(const LinearBwdArgs& a, const HostSegs& hs, cudaStream_t st) {
+    const unsigned split = (unsigned)bias_split(a.n_rows, a.n_expert, a.out_feat);
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)ceil_div(a.out_feat, 128), (unsigned)a.n_expert, kBiasSplit);
+    cfg.gridDim = dim3((unsigned)ceil_div(a.out_feat, 128), (unsigned)a.n_expert, split);
     cfg.blockDim = dim3(256);
     cfg.stream = st;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = 1; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = kBiasSplit;
+    attr[0].val.clusterDim.x = 1; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = split;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = split > 1 ? 1 : 0;
     FMOE_CUDA_TRY(cudaLaunchKernelEx(&cfg, bias_grad_tc_kernel<BF16>, (const uint16_t*)a.grad_y, a.seg_offsets, hs,
                                      (uint16_t*)a.grad_b, a.n_rows, (int)a.out_feat, a.accumulate));
     return 0;
@@ -1861,6 +1885,68 @@ int tc_linear_forward(const LinearArgs& a, cudaStream_t st) {
                 : launch<MODE_FWD, false>(ma, mb, a.host_segs, p, max_tiles, a.n_rows, st, reserve, a.remote, a.push);
 }
 
+// The bias gradient (a column sum bound by HBM, with a small footprint) of 16 MB of rows and more runs beside the products of
+// the same call, on a side stream of the device that is created on first use: whole backward of one expert with 4096 rows,
+// 1024 x 4096, 83 us in stream order and 74 beside the products; 16 experts with 1024 rows each, 1024 x 4096, 267 and 254.
+// With fewer rows the kernel is short (3-7 us in stream order) and the four stream operations cost the host more than
+// that: step of 3001 tokens, 12 experts of 768 x 3072, 9 MB: 530 us with them, 516 without.
+// Threads share the stream and its events: a fork and its kernel are queued under the lock, and a join that another thread
+// has recorded again only waits for later work of the same stream.  A call under capture stays in stream order: the
+// side stream must not be drawn into one caller's capture while others use it.
+constexpr int64_t kBranchElements = 8 << 20;      // 16 MB
+struct SideStream {
+    cudaStream_t stream = nullptr;
+    cudaEvent_t fork = nullptr, join = nullptr;
+};
+struct BiasBranch {
+    cudaStream_t st;
+    SideStream* side = nullptr;
+    std::unique_lock<std::mutex> lock;
+    bool open = false;
+
+    int fork(cudaStream_t* on) {
+        static SideStream pool[64];
+        static std::mutex mtx;
+        cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+        int dev = 0;
+        if (cudaStreamIsCapturing(st, &capture) != cudaSuccess) { cudaGetLastError(); return 0; }
+        if (capture != cudaStreamCaptureStatusNone) return 0;
+        FMOE_CUDA_TRY(cudaGetDevice(&dev));
+        if (dev < 0 || dev >= 64) return 0;
+        lock = std::unique_lock<std::mutex>(mtx);
+        SideStream& s = pool[dev];
+        if (!s.join) {
+            // (another thread may be capturing: creating these concerns no stream of its graph)
+            cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+            FMOE_CUDA_TRY(cudaThreadExchangeStreamCaptureMode(&mode));
+            cudaError_t err = s.stream ? cudaSuccess : cudaStreamCreateWithFlags(&s.stream, cudaStreamNonBlocking);
+            if (err == cudaSuccess && !s.fork) err = cudaEventCreateWithFlags(&s.fork, cudaEventDisableTiming);
+            if (err == cudaSuccess) err = cudaEventCreateWithFlags(&s.join, cudaEventDisableTiming);
+            FMOE_CUDA_TRY(cudaThreadExchangeStreamCaptureMode(&mode));
+            FMOE_CUDA_TRY(err);
+        }
+        FMOE_CUDA_TRY(cudaEventRecord(s.fork, st));
+        FMOE_CUDA_TRY(cudaStreamWaitEvent(s.stream, s.fork, 0));
+        side = &s;
+        *on = s.stream;
+        return 0;
+    }
+    int record() {
+        if (!side) return 0;
+        FMOE_CUDA_TRY(cudaEventRecord(side->join, side->stream));
+        open = true;
+        lock.unlock();
+        return 0;
+    }
+    int join() {
+        if (!open) return 0;
+        open = false;
+        FMOE_CUDA_TRY(cudaStreamWaitEvent(st, side->join, 0));
+        return 0;
+    }
+    ~BiasBranch() { if (open) cudaStreamWaitEvent(st, side->join, 0); }     // a call that failed half-way
+};
+
 int tc_linear_backward(const LinearBwdArgs& a, cudaStream_t st) {
     const bool bf16 = a.dtype == FMOE_BF16;
     const HostSegs& hs = a.host_segs ? *a.host_segs : kNoSegs;
@@ -1872,11 +1958,13 @@ int tc_linear_backward(const LinearBwdArgs& a, cudaStream_t st) {
         if (a.after_input_grad) { if (int rc = a.after_input_grad(a.after_ctx)) return rc; }
         closed = true;
     }
-    // The bias gradient comes first, while L2 still holds part of the rows the caller has just written.  (On a stream
-    // of its own beside the products, it got its SMs only when the persistent input-gradient product gave them up, and
-    // then kept the weight gradient from them.)
+    BiasBranch branch{st};
     auto bias_grad = [&]() -> int {
-        return !a.grad_b ? 0 : bf16 ? launch_bias_grad<true>(a, hs, st) : launch_bias_grad<false>(a, hs, st);
+        if (!a.grad_b) return 0;
+        cudaStream_t on = st;
+        if ((a.grad_x || a.grad_w) && a.n_rows * a.out_feat >= kBranchElements) { if (int rc = branch.fork(&on)) return rc; }
+        if (int rc = bf16 ? launch_bias_grad<true>(a, hs, on) : launch_bias_grad<false>(a, hs, on)) return rc;
+        return branch.record();
     };
     if (closed) { if (int rc = bias_grad()) return rc; }
     if (a.grad_x && a.n_rows > 0) {
@@ -1953,7 +2041,7 @@ int tc_linear_backward(const LinearBwdArgs& a, cudaStream_t st) {
                           : launch<MODE_WGRAD, false>(ma, mb, a.host_segs, p, max_tiles, (int64_t)a.n_expert * a.out_feat, st, reserve))
             return rc;
     }
-    return 0;
+    return branch.join();
 }
 
 int* device_status_ptr() { return status_ptr(); }

@@ -505,3 +505,71 @@ def test_token_minor_activations(fc, form, dtype, act):
             close(pre[p:p + c], torch.autograd.grad(fn(z).sum(), z)[0])
         close(gx[p:p + c], gy[p:p + c].float() @ w[e].float() * factor[p:p + c])
         p += c
+
+
+BIAS_GRADIENTS = [
+    # rows of the experts (long and empty ones among them), out_feat: every number of blocks that share a segment
+    ([20] * 100, 4096),                         # one block
+    ([140] * 15 + [0], 4096),                   # two, beside the products
+    ([1] + [320] * 14 + [0], 4096),             # four, beside the products
+    ([3, 0, 40, 1], 320),                       # eight, most of them without rows
+    ([9000, 5, 0], 128),                        # eight, rows that eight does not divide; out_feat off the grid
+]
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("counts,fout", BIAS_GRADIENTS)
+def test_bias_gradient(fc, dtype, counts, fout):
+    """Column sums per segment against fp64: fp32 sums of 16-bit rows, rounded once; the same from call to call, beside the
+    products and (in a captured graph) in stream order before them."""
+    from fastermoe_b200 import _lib
+    E, B, fin = len(counts), sum(counts), 256
+    off = torch.tensor(np.concatenate([[0], np.cumsum(counts)]), dtype=torch.int64, device="cuda")
+    x, gy = torch.randn(B, fin, device="cuda").to(dtype), torch.randn(B, fout, device="cuda").to(dtype)
+    w = (torch.randn(E, fout, fin, device="cuda") / np.sqrt(fout)).to(dtype)
+    runs = [fc.linear_backward_act(gy, x, off, w, None, _lib.ACT_NONE)[2] for _ in range(3)]
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        captured = fc.linear_backward_act(gy, x, off, w, None, _lib.ACT_NONE)[2]
+    graph.replay()
+    assert all(torch.equal(r, captured) for r in runs)
+    eps = torch.finfo(dtype).eps
+    p = 0
+    for e, c in enumerate(counts):
+        rows = gy[p:p + c].double()
+        # one rounding to the output type, and c fp32 additions of terms whose magnitudes add up to `size`
+        want, size = rows.sum(0), rows.abs().sum(0)
+        bound = 0.5 * eps * want.abs() + (c + 1) * 2.0 ** -24 * size * (1 + eps)
+        assert bool(((captured[e].double() - want).abs() <= bound).all())
+        p += c
+
+
+def test_bias_gradient_from_threads(fc):
+    """Two threads on streams of their own, their backward calls interleaved: the side stream that they share takes each
+    gradient after its rows and before it is read."""
+    import threading
+    from fastermoe_b200 import _lib
+    E, B, fin, fout = 4, 4096, 256, 512
+    off = torch.arange(0, B + 1, B // E, device="cuda")
+    w = torch.randn(E, fout, fin, device="cuda").bfloat16()
+    torch.cuda.synchronize()
+    wrong = []
+
+    def work(seed):
+        stream = torch.cuda.Stream()
+        g = torch.Generator(device="cuda").manual_seed(seed)
+        with torch.cuda.stream(stream):
+            x = torch.randn(B, fin, device="cuda", generator=g).bfloat16()
+            for _ in range(30):
+                gy = torch.randint(-4, 5, (B, fout), device="cuda", generator=g).bfloat16()      # sums are exact in fp32
+                gb = fc.linear_backward_act(gy, x, off, w, None, _lib.ACT_NONE)[2]
+                want = gy.float().view(E, B // E, fout).sum(1).bfloat16()
+                wrong.append((gb != want).sum())
+            stream.synchronize()
+
+    threads = [threading.Thread(target=work, args=(s,)) for s in (1, 2)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert len(wrong) == 60 and int(torch.stack(wrong).sum()) == 0
