@@ -1712,9 +1712,11 @@ bias_grad_tc_kernel(const uint16_t* __restrict__ dy, const int64_t* __restrict__
 // Adds up the per-block partial column sums that the input-gradient kernel left in the
 // scratch buffer: out[e, col] = sum over the 32-row blocks of expert e.  Four thread rows
 // take a quarter of the blocks each (in block order) and the quarters are added in order,
-// so the result does not depend on timing.
+// so the result does not depend on timing.  Three blocks per SM leave a thread registers for eight loads in flight; held to
+// 32 registers for a fourth block, it waits for them two at a time (two experts of 16384 rows, 16384 columns: 82 us, 27
+// here; 16 of 2048, 4096 columns: 12.2 and 6.8; 32 skewed ones, 8192 columns: 22 and 12; 64 of 8 rows: 11 and 11-13).
 template <bool BF16>
-__global__ void __launch_bounds__(512)
+__global__ void __launch_bounds__(512, 3)
 colsum_finish_kernel(const float* __restrict__ partial, const int64_t* __restrict__ seg, const __grid_constant__ HostSegs hs,
                      uint16_t* __restrict__ out, int64_t n_rows, int n_cols, int accumulate) {
     __shared__ float2 part[4][128];
