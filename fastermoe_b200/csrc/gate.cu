@@ -226,7 +226,18 @@ namespace fmoe {
 namespace {
 
 constexpr int kBalMax = 256, kBalRegs = kBalMax / 32, kBalWarps = 8;
-int balance_blocks(int64_t n_tokens) { return (int)std::min<int64_t>(ceil_div(n_tokens, kBalWarps), 128); }
+
+// Threads of the finishing block per expert: what is left of kBalMax when the experts are rounded up to a power of two.
+__host__ __device__ constexpr int balance_parts(int n_expert) {
+    int w = 1;
+    while (w < n_expert) w *= 2;
+    return kBalMax / w;
+}
+// Blocks of the summing kernel: a block per eight tokens, as many as the finishing threads add in 128 steps each, at most 512
+// (131072 tokens, 16 experts, loss and gradient: 158 us with 128 blocks and one finishing thread per expert, 86 here).
+int balance_blocks(int64_t n_tokens, int n_expert) {
+    return (int)std::min<int64_t>(ceil_div(n_tokens, kBalWarps), 128 * std::min(balance_parts(n_expert), 4));
+}
 
 // softmax of one row; the lanes' shares of it (zero past n_expert)
 template <typename T>
@@ -290,24 +301,31 @@ balance_sums_kernel(const T* __restrict__ logits, const int64_t* __restrict__ fi
 __global__ void __launch_bounds__(kBalMax)
 balance_finish_kernel(const float* __restrict__ partial, const int* __restrict__ counts, int blocks, int64_t n_tokens,
                       int n_expert, float scale, float* __restrict__ loss, float* __restrict__ share) {
-    __shared__ float terms[kBalMax];
-    const int e = threadIdx.x;
-    float term = 0.f;
+    __shared__ float terms[kBalMax], sums[kBalMax];
+    __shared__ int hits[kBalMax];
+    const int parts = balance_parts(n_expert), width = kBalMax / parts, e = threadIdx.x % width, part = threadIdx.x / width;
+    float s = 0.f;
+    int c = 0;
     if (e < n_expert) {
-        float s = 0.f;
-        int c = 0;
 #pragma unroll 8
-        for (int b = 0; b < blocks; ++b) {
+        for (int b = part; b < blocks; b += parts) {
             s += partial[(size_t)b * n_expert + e];
             c += counts[(size_t)b * n_expert + e];
         }
-        const float part = (float)c / (float)n_tokens;
-        share[e] = part;
-        term = part * (s / (float)n_tokens);
     }
-    terms[e] = term;
+    sums[threadIdx.x] = s;
+    hits[threadIdx.x] = c;
     __syncthreads();
-    if (e == 0) {
+    float term = 0.f;
+    if (part == 0 && e < n_expert) {
+        for (int q = 1; q < parts; ++q) { s += sums[q * width + e]; c += hits[q * width + e]; }
+        const float f = (float)c / (float)n_tokens;
+        share[e] = f;
+        term = f * (s / (float)n_tokens);
+    }
+    terms[threadIdx.x] = term;       // (zero for the parts after the first)
+    __syncthreads();
+    if (threadIdx.x == 0) {
         float t = 0.f;
         for (int i = 0; i < n_expert; ++i) t += terms[i];
         *loss = t * scale;
@@ -351,7 +369,7 @@ int check_balance(const void* logits, int64_t n_tokens, int32_t n_expert, int32_
 }  // namespace fmoe
 
 extern "C" size_t fmoe_balance_loss_scratch_bytes(int64_t n_tokens, int32_t n_expert) {
-    return n_tokens > 0 && n_expert > 0 ? (size_t)balance_blocks(n_tokens) * (size_t)n_expert * 8 : 0;
+    return n_tokens > 0 && n_expert > 0 ? (size_t)balance_blocks(n_tokens, n_expert) * (size_t)n_expert * 8 : 0;
 }
 
 extern "C" int fmoe_balance_loss(const void* logits, const int64_t* first_choice, int64_t choice_stride, int64_t n_tokens,
@@ -360,7 +378,7 @@ extern "C" int fmoe_balance_loss(const void* logits, const int64_t* first_choice
     if (int rc = check_balance(logits, n_tokens, n_expert, dtype)) return rc;
     FMOE_REQUIRE(first_choice && loss && share && scratch, "balance_loss: null pointer");
     cudaStream_t st = (cudaStream_t)stream;
-    const int blocks = balance_blocks(n_tokens);
+    const int blocks = balance_blocks(n_tokens, n_expert);
     float* partial = (float*)scratch;
     int* counts = (int*)scratch + (size_t)blocks * n_expert;
     switch (dtype) {

@@ -338,3 +338,21 @@ def test_silu_with_a_strided_weight(dtype):
     tol = 1e-5 if dtype == torch.float32 else 2e-2
     for a, b in zip(step(m, x, g), want):
         assert float((a.double() - b.double()).norm()) <= tol * float(b.double().norm())
+
+
+@pytest.mark.parametrize("T,E", [(5000, 2), (70000, 16), (9001, 64), (3000, 65), (4097, 256)])
+def test_balance_loss_of_many_tokens(T, E):
+    """Every number of blocks, and of finishing threads per expert, that the sizes select, against the definition in fp64.
+    An element of the gradient is p (w - sum p w): its error is a few roundings of the largest w, whatever cancels."""
+    from fastermoe_b200.gates.gshard_gate import balance_loss_top1
+    logits = torch.randn(T, E, device="cuda", requires_grad=True)
+    idx = torch.randint(0, E, (T,), device="cuda")
+    loss = balance_loss_top1(idx, logits, E, E)
+    loss.backward()
+    ref = logits.detach().double().requires_grad_(True)
+    share = torch.bincount(idx, minlength=E).double() / T
+    want = (share * torch.softmax(ref, 1).mean(0)).mean() * E ** 2
+    want.backward()
+    assert abs(float(loss.detach()) - float(want.detach())) <= 1e-5 * float(want.detach())
+    w = E * share / T
+    torch.testing.assert_close(logits.grad.double(), ref.grad, rtol=1e-5, atol=8 * 2.0 ** -23 * float(w.max()))
