@@ -87,7 +87,17 @@ topk_forward_kernel(const T* __restrict__ logits, int64_t n_tokens, int n_expert
             indices[tok * k + j] = vi;
         }
     }
-    if (SOFTMAX && lane == 0) store_softmax<T>(won, k, values + tok * k);
+    if (SOFTMAX) {          // all lanes know the winners: each stores one probability (131072 x 256, k = 8: 252 us by one lane, 241)
+        float mine = 0.f, sum = 0.f;
+#pragma unroll
+        for (int j = 0; j < kTopKMax; ++j)
+            if (j < k) {
+                const float p = expf(won[j] - won[0]);
+                sum += p;
+                if (j == lane) mine = p;
+            }
+        if (lane < k) values[tok * k + lane] = from_float<T>(mine / sum);
+    }
 }
 
 // Few experts (<= 32): one THREAD per token; a warp then reads 32 consecutive rows, i.e. one
